@@ -174,6 +174,8 @@ struct Context {
     uint32_t max_mesh_height = 0;
 
     DevArray<float4> d_geometries, d_scene_nodes, d_mesh_nodes, d_tri_hot, d_tri_cold;
+    DevArray<WideNode> d_wide_nodes;
+    DevArray<WideLeaf> d_wide_leaves;
     DevArray<SlimMaterial> d_materials;
     DevArray<SlimLight> d_lights;
     DevArray<uint32_t> d_leaf_geometry, d_emissive_quads, d_refit_order;
@@ -513,14 +515,17 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
 
     int rc = c.d_meshes.reserve(metas.size(), "alloc meshes");
     if (rc) return rc;
-    SLIM_CUDA(cudaMemcpy(c.d_meshes.ptr, metas.data(), metas.size() * sizeof(DevMesh), cudaMemcpyHostToDevice), "upload meshes");
     c.scene.meshes = c.d_meshes.ptr;
     c.scene.mesh_count = n;
     if (!n) {
         c.scene.mesh_nodes = nullptr;
         c.scene.tri_hot = c.scene.tri_cold = nullptr;
+        c.scene.wide_nodes = nullptr;
+        c.scene.wide_leaves = nullptr;
         return SLIM_OK;
     }
+    std::vector<WideNode> wide;
+    std::vector<WideLeaf> wide_leaves;
     rc = c.d_mesh_nodes.reserve(2 * total_nodes, "alloc mesh nodes");
     if (rc) return rc;
     rc = c.d_tri_hot.reserve(3 * total_tris, "alloc triangles");
@@ -530,7 +535,7 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
     std::vector<float4> hot, cold;
     for (uint32_t i = 0; i < n; i++) {
         const SlimMesh &m = s->meshes[i];
-        const DevMesh &dm = metas[i];
+        DevMesh &dm = metas[i];
         SLIM_CUDA(cudaMemcpy(c.d_mesh_nodes.ptr + 2 * (size_t)dm.node_offset, m.bvh.nodes, m.bvh.node_count * sizeof(SlimBVHNode),
                              cudaMemcpyHostToDevice), "upload mesh nodes");
         hot.resize(3 * (size_t)m.triangle_count);
@@ -550,7 +555,20 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
                              cudaMemcpyHostToDevice), "upload triangles");
         SLIM_CUDA(cudaMemcpy(c.d_tri_cold.ptr + 4 * (size_t)dm.tri_offset, cold.data(), cold.size() * sizeof(float4),
                              cudaMemcpyHostToDevice), "upload triangle attributes");
+        dm.wide_root = build_wide_bvh(m.bvh.nodes, m.bvh.node_count, &hot[0].x, kStackCapacity, wide, wide_leaves,
+                                      dm.wide_extent);
     }
+    SLIM_CUDA(cudaMemcpy(c.d_meshes.ptr, metas.data(), metas.size() * sizeof(DevMesh), cudaMemcpyHostToDevice), "upload meshes");
+    if ((rc = c.d_wide_nodes.reserve(wide.size() ? wide.size() : 1, "alloc wide nodes"))) return rc;
+    if ((rc = c.d_wide_leaves.reserve(wide_leaves.size() ? wide_leaves.size() : 1, "alloc wide leaves"))) return rc;
+    if (!wide.empty()) {
+        SLIM_CUDA(cudaMemcpy(c.d_wide_nodes.ptr, wide.data(), wide.size() * sizeof(WideNode), cudaMemcpyHostToDevice),
+                  "upload wide nodes");
+        SLIM_CUDA(cudaMemcpy(c.d_wide_leaves.ptr, wide_leaves.data(), wide_leaves.size() * sizeof(WideLeaf),
+                             cudaMemcpyHostToDevice), "upload wide leaves");
+    }
+    c.scene.wide_nodes = reinterpret_cast<const uint4 *>(c.d_wide_nodes.ptr);
+    c.scene.wide_leaves = reinterpret_cast<const float4 *>(c.d_wide_leaves.ptr);
     c.scene.mesh_nodes = c.d_mesh_nodes.ptr;
     c.scene.tri_hot = c.d_tri_hot.ptr;
     c.scene.tri_cold = c.d_tri_cold.ptr;

@@ -5,6 +5,8 @@
 //   geometry       4 x float4   rotation quat | position,type | scale,material | 1/scale,flags+mesh
 //   BVH node       2 x float4   the reference's 32-byte BVHNode bytes unchanged
 //                               (min.xyz, max.x | max.yz, first_index, leaf_count/depth/flags)
+//   wide node      5 x uint4    four children's boxes, for the persistent mesh walks (wide_bvh.h)
+//   wide leaf      8 x float4   a leaf's BVH node and the hot bytes of its first two triangles
 //   triangle hot   3 x float4   position, normal and the two rows of local_to_tangent
 //                               the hit test reads (48 B of the reference's 128 B)
 //   triangle cold  4 x float4   n1..n3, uv1..uv3, uv_coverage (read once per mesh hit)
@@ -15,15 +17,15 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "slimtracer_b200.h"
+#include "wide_bvh.h"
 
 namespace slim {
 
-constexpr int kStackCapacity = 64;
-// Mesh-BVH leaves waiting in the persistent mesh kernels are packed as
-// first triangle | count << kLeafCountShift: meshes hold fewer than 2^26
-// triangles and leaves below the root fewer than 64 (checked on upload; the
-// reference's builder makes leaves of at most two).
-constexpr uint32_t kLeafCountShift = 26;        // per-ray traversal stack entries (scene and mesh)
+constexpr int kStackCapacity = 64;        // per-ray traversal stack entries (scene and mesh)
+// Meshes hold fewer than 2^26 triangles and leaves below the root fewer than
+// 64 (checked on upload; the reference's builder makes leaves of at most
+// two).
+constexpr uint32_t kLeafCountShift = 26;
 constexpr int kMaxLights = 64;            // lights a shadow mask can track
 constexpr uint32_t kErrStack = 1u;        // device error bits
 constexpr uint32_t kErrIndex = 2u;
@@ -35,6 +37,8 @@ struct DevMesh {
     uint32_t tri_count;
     uint32_t node_count;
     uint32_t has_normals, has_uvs;
+    uint32_t wide_root;       // into wide_nodes, or kNoWideBVH
+    float wide_extent;        // bound of its planes (wide_bvh.h)
 };
 
 struct DevMip {
@@ -59,6 +63,8 @@ struct DevScene {
     const float4 *mesh_nodes;
     const float4 *tri_hot;
     const float4 *tri_cold;
+    const uint4 *wide_nodes;       // 5 per node of the four-wide mesh BVHs (wide_bvh.h)
+    const float4 *wide_leaves;     // 8 per leaf record
     const DevTexture *textures;
     const DevMip *mips;
     const uint4 *quads;

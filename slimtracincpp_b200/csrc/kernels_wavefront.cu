@@ -23,6 +23,7 @@
 #include "kernels.h"
 #include "nrc.h"
 #include "tracer_core.cuh"
+#include "wide_bvh.cuh"
 
 namespace slim {
 namespace dev {
@@ -116,7 +117,7 @@ struct QueueArgs {
     uint32_t *shadow_count;
     unsigned long long *masks;    // per slot: bit i = light i occluded
     float4 *pairs;                // shadow ray x mesh instance candidates, 3 float4 each:
-                                  // (local origin, aux distance) (local direction, tag) (nodes, triangles, first child)
+                                  // (local origin, aux distance) (local direction, tag) (wide root, triangles, plane bound, 0)
     uint32_t *pair_count;
     uint32_t *pair_cursor;
     uint32_t pair_capacity;
@@ -295,10 +296,11 @@ __global__ void __launch_bounds__(256) k_shadow_gen(DevScene S0, DevFrame F0, Qu
 //   shadow_scene  walks the scene BVH per shadow ray, tests implicit
 //                 primitives on the spot and appends one (ray, mesh
 //                 instance, aux distance) pair per reached mesh instance;
-//   shadow_mesh   a persistent kernel (leaves parked, see PendingLeaves) in which every lane runs one mesh BVH
-//                 traversal step per loop turn and fetches the next pair as
-//                 soon as its own finishes, so warps stay full although
-//                 traversal lengths differ by orders of magnitude.
+//   shadow_mesh   a persistent kernel in which every lane visits a node or
+//                 two of a mesh's four-wide BVH per loop turn, lets a leaf
+//                 wait until enough lanes have one, and fetches the next
+//                 pair as soon as its own finishes, so warps stay full
+//                 although walk lengths differ by orders of magnitude.
 
 SLIM_D bool local_box_test(const DevScene &S, const Geo &g, const Ray &local) {
     float mn[3], mx[3], n, f;
@@ -350,15 +352,15 @@ SLIM_D bool shadow_leaf(const DevScene &S, const QueueArgs &A, uint32_t tag, uin
                     if (hit_triangles<COUNT>(S.tri_hot, m.tri_offset, m.tri_count, lf2, local, h, true, w)) return true;
                     break;
                 }
-                uint32_t slot = warp_append(A.pair_count, true);
-                if (slot < A.pair_capacity) {
+                const bool wide = m.wide_root != kNoWideBVH;
+                uint32_t slot = warp_append(A.pair_count, wide);
+                if (wide && slot < A.pair_capacity) {
                     float4 *p = A.pairs + 3 * (size_t)slot;
                     p[0] = make_float4(local.o.x, local.o.y, local.o.z, aux);
                     p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(tag));
-                    p[2] = make_float4(__uint_as_float(m.node_offset), __uint_as_float(m.tri_offset),
-                                       __uint_as_float(node_first(rb)), 0.0f);
+                    p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
                 } else if (mesh_trace<COUNT>(S, m, local, h, true, mesh_stack, err, w)) {
-                    return true;   // pair queue full: trace the instance here
+                    return true;   // no wide walk, or the pair queue is full: trace the instance here
                 }
             } break;
             default: break;
@@ -439,64 +441,40 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
 }
 
 
-// Leaves a walk reaches wait (up to three per lane, in visiting order) while
-// the lane keeps stepping through inner nodes; the warp tests triangles only
-// when enough of its lanes have a waiting leaf (kLeafFraction) or none can
-// step, so the triangle code runs with many lanes busy instead of one or two.
-// A lane keeps stepping through inner nodes while at most kStepWhileWaiting
-// leaves wait (config 2: stepping with one leaf waiting 2.03 -> 1.94 ms).
-constexpr uint32_t kStepWhileWaiting = 1;
-// Inner steps a walking lane takes per loop turn: the turn's warp votes (new
-// candidates? leaf tests?) are paid once per two steps (config 2: 1.55 ->
-// 1.48 ms; three steps measured the same as two).
+// The persistent mesh walks.  They run over the four-wide form of the mesh
+// BVHs (wide_bvh.h).  What bounds them is instructions issued at 14-18 busy
+// lanes of 32, then the L1 bytes of the nodes (each lane at its own), so the
+// form was chosen by both, on the 1080p frame of the 81,920- and
+// 130,050-triangle meshes (any-hit launch of the first round, ncu):
+//   two-wide, 64 B a step, 24.4 steps per walk        281 M warp instr., 385 us
+//   eight-wide, 8-bit planes, 80 B, 9.0 nodes         238 M, L1 50 %, 321 us
+//   four-wide, 32-bit planes, 112 B read, 13 nodes    169 M, L1 83 %, 328 us
+//   four-wide, 16-bit planes, 80 B, 11.7 nodes        201 M, L1 67 %, 292 us (this)
+// (the last also goes to the child that reaches furthest first).  The frame:
+// 1.455 -> 1.283 ms; with 8 bounces 2.865 -> 2.550 ms.
+//
+// Nodes a walking lane visits per loop turn: with one 1.35, three 1.38
+// against 1.29 ms.
 constexpr uint32_t kStepsPerTurn = 2;
-// kStepWhileWaiting + 2 slots: a lane steps only with at most
-// kStepWhileWaiting leaves waiting, and a step adds at most two.  A waiting
-// leaf is packed into one word, first triangle | count << kLeafCountShift
-// (mesh uploads are limited to fit), which frees registers for the walk
-// (config 2: 1.45 -> 1.44 ms).
-struct PendingLeaves {
-    uint32_t leaf0, leaf1, leaf2;
-    float clip0, clip1, clip2;
-    uint32_t n;
-    uint32_t first0, count0;            // slot 0 unpacked
-    SLIM_D void push(uint32_t f, uint32_t c, float far) {
-        const uint32_t v = f | (c << kLeafCountShift);
-        if (n == 0) { leaf0 = v; clip0 = far; }
-        else if (n == 1) { leaf1 = v; clip1 = far; }
-        else { leaf2 = v; clip2 = far; }
-        n++;
-        unpack();
-    }
-    SLIM_D void pop() {
-        leaf0 = leaf1; clip0 = clip1;
-        leaf1 = leaf2; clip1 = clip2;
-        n--;
-        unpack();
-    }
-    SLIM_D void unpack() {
-        first0 = leaf0 & ((1u << kLeafCountShift) - 1u);
-        count0 = leaf0 >> kLeafCountShift;
-    }
-    SLIM_D bool can_step() const { return n <= kStepWhileWaiting; }
-};
-static_assert(kStepWhileWaiting + 2 <= 3, "PendingLeaves holds three leaves");
 
 // Warp-uniform decision: should idle lanes take new candidates now?  Idle
-// lanes wait until a quarter of the warp is idle (or nobody is busy) and
+// lanes wait until a third of the warp is idle (or nobody is busy) and
 // then fetch together, so the fetch code -- one atomic, the candidate loads,
 // the ray set-up -- runs for several lanes at once instead of for the one or
 // two that finished this turn (config 2: 1.94 -> 1.82 ms).
-constexpr uint32_t kFetchFraction = 4;   // fetch when idle lanes >= active lanes / kFetchFraction
+constexpr uint32_t kFetchFraction = 3;   // fetch when idle lanes >= active lanes / kFetchFraction
 SLIM_D bool fetch_round(bool idle) {
     const uint32_t act = __activemask();
     const uint32_t idle_mask = __ballot_sync(act, idle);
     return idle_mask && (kFetchFraction * (uint32_t)__popc(idle_mask) >= (uint32_t)__popc(act) || idle_mask == act);
 }
 
+// No node: as a reference it counts as a leaf, so no lane steps into it.
+constexpr uint32_t kNone = 0xFFFFFFFFu;
+
 // Warp-uniform decision: test waiting leaves now?  Once a third of the warp
-// has a leaf waiting, or no lane can step (with two steps per turn, a third
-// measured 1.49 -> 1.47 ms on config 2 against a half).
+// has a leaf waiting, or no lane can step (1.291 ms; a half or a quarter
+// 1.296).
 constexpr uint32_t kLeafFraction = 3;
 SLIM_D bool leaf_round(bool waiting, bool can_step) {
     const uint32_t act = __activemask();
@@ -505,17 +483,13 @@ SLIM_D bool leaf_round(bool waiting, bool can_step) {
     return wait_mask && (kLeafFraction * (uint32_t)__popc(wait_mask) >= (uint32_t)__popc(act) || !step_mask);
 }
 
-// The persistent mesh kernels run 128-thread blocks with a register cap
-// that fits one more block per SM than their natural use (shadow: 61 -> 56
-// registers, 32 -> 36 warps per SM; closest hit: 73 -> 70 registers, 24 -> 28
-// warps): their walks wait on dependent loads, so warps beat registers
-// (config 2: 1.61 -> 1.57 ms with the closest-hit pass, 1.59 with the any-hit
-// pass alone).  With the later walk changes, config 2 at 9 / 7 blocks takes
-// 1.437-1.443 ms; 10 or 12 any-hit blocks 1.54 / 1.68 ms (spills), 8 or 9
-// closest-hit blocks 1.48-1.49 ms.
+// 128-thread blocks, capped at 64 registers for the any-hit walks (32 warps
+// per SM) and 72 for the closest-hit walks (28): 1.284 ms; any hit at 9 or
+// 10 blocks 1.291 and 1.448 ms (spills), closest hit at 6 or 8 blocks 1.307
+// and 1.292 ms.
 constexpr int kMeshBlock = 128;
 #ifndef SLIM_SHADOW_MESH_BLOCKS
-#define SLIM_SHADOW_MESH_BLOCKS 9
+#define SLIM_SHADOW_MESH_BLOCKS 8
 #endif
 #ifndef SLIM_EXTEND_MESH_BLOCKS
 #define SLIM_EXTEND_MESH_BLOCKS 7
@@ -528,11 +502,8 @@ constexpr int kMeshBlock = 128;
 // of running one lane each while the rest of the warp waits.  The i-th idle
 // lane (in lane order) takes from the i-th lane with a pending subtree; the
 // giver removes the entry from its stack.  Exact: an any-hit result is the
-// OR over the leaves a walk reaches, whatever the order (config 2: 1.46 ->
-// 1.45 ms; config 4's plain depth-8 frame, whose late rounds are almost all
-// tail: 3.00 -> 2.91 ms).  The closest-hit walks do not share: a piece that
-// does not know the best hit of the part before it in the reference's order
-// could report a triangle the reference culls.
+// OR over the leaves a walk reaches, whatever the order (1.46 -> 1.45 ms;
+// with 8 bounces, whose late rounds are almost all tail, 3.00 -> 2.91 ms).
 struct Steal {
     int from;           // giving lane for a taker, else -1
     uint32_t subtree;   // stack entry handed over (valid for a taker)
@@ -557,48 +528,71 @@ SLIM_D Steal steal_round(uint32_t act, uint32_t idle_mask, uint32_t donor_mask, 
     st.from = taker ? src : -1;
     return st;
 }
-// Stack push for walks that may give entries away from the bottom: the live
-// entries are [bottom, top); when the top reaches the capacity they move
-// down first.  Returns false on overflow.
-SLIM_D bool push_entry(uint32_t *stack, uint32_t &bottom, uint32_t &top, uint32_t v) {
-    if (top >= (uint32_t)kStackCapacity) {
-        if (bottom == 0) return false;
-        for (uint32_t i = bottom; i < top; i++) stack[i - bottom] = stack[i];
-        top -= bottom;
-        bottom = 0;
+
+// The hot record of triangle i of a leaf whose first triangle is `first`:
+// the first two lie in the leaf's own line.
+SLIM_D const float4 *leaf_triangle(const DevScene &S, const float4 *leaf, uint32_t first, uint32_t i) {
+    return i < 2 ? leaf + 2 + 3 * i : S.tri_hot + 3 * (size_t)(first + i);
+}
+
+// MeshTracer::hitTriangles (mesh_tracer.h:23-49) over a wide leaf, any hit
+// closer than `closest`.
+template <bool COUNT>
+SLIM_D bool any_triangle(const DevScene &S, const float4 *leaf, uint32_t tri_offset, float4 node, float closest,
+                         const Ray &r, Work &w) {
+    const uint32_t count = node_leaf_count(node), first = tri_offset + node_first(node);
+    for (uint32_t i = 0; i < count; i++) {
+        bump<COUNT>(w.triangles);
+        const float4 *t4 = leaf_triangle(S, leaf, first, i);
+        const float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
+        const float3 p = xyz(a), n = f3(a.w, b.x, b.y);
+        float t; float3 pos; bool behind;
+        if (!hit_plane(r, p, n, t, pos, behind)) continue;
+        const float3 q = pos - p;
+        const float ux = b.z * q.x + c.x * q.y + c.z * q.z;
+        const float uy = b.w * q.x + c.y * q.y + c.w * q.z;
+        if (!(ux < 0 || uy < 0 || (ux + uy) > 1 || t >= closest)) return true;
     }
-    stack[top++] = v;
-    return true;
+    return false;
 }
 
 template <bool COUNT>
 __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_mesh(DevScene S, DevFrame F, QueueArgs A) {
     const uint32_t n = *A.pair_count < A.pair_capacity ? *A.pair_count : A.pair_capacity;
     uint32_t stack[kStackCapacity];
-    uint32_t err = 0;
     Work w = {};
-    bool busy = false, walking = false, drained = false;
-    uint32_t idx = 0, tag = 0, left = 0, top = 0, bottom = 0, tri_offset = 0;
-    const float4 *nodes = nullptr;
+    bool busy = false, drained = false;
+    uint32_t idx = 0, tag = 0, top = 0, bottom = 0, tri_offset = 0;
+    uint32_t next = kNone;          // node or leaf the walk goes to
+    uint32_t waiting = kNone;       // a leaf to be tested
     float aux = 0.0f;
     Ray r;
-    PendingLeaves pend;
-    pend.n = 0;
-    // (shadow ray, instance) pair i from its root's children, or from `subtree`
-    auto start = [&](uint32_t i, uint32_t subtree, bool whole) {
+    WideRay wr;
+    // Where the walk goes after a node or a leaf: a leaf waits while the walk
+    // goes on, so that `next` is a leaf only while another one waits.
+    auto advance = [&]() {
+        if (next == kNone && top > bottom) next = stack[--top];
+        if (next != kNone && (next & kWideLeaf) && waiting == kNone) {
+            waiting = next;
+            next = top > bottom ? stack[--top] : kNone;
+        }
+    };
+    // (shadow ray, instance) pair i from its root, or from a node of its walk
+    auto start = [&](uint32_t i, uint32_t from) {
         const float4 *p = A.pairs + 3 * (size_t)i;
         float4 p0 = p[0], p1 = p[1], p2 = p[2];
         tag = __float_as_uint(p1.w);
         if ((A.masks[tag >> 6] >> (tag & 63u)) & 1ull) return;   // already known occluded
         idx = i;
         reset(r, xyz(p0), xyz(p1));
+        wr = wide_setup(r, p2.z);
         aux = p0.w;
-        nodes = S.mesh_nodes + 2 * (size_t)__float_as_uint(p2.x);
         tri_offset = __float_as_uint(p2.y);
-        left = whole ? __float_as_uint(p2.z) : subtree;
+        next = from == kNone ? __float_as_uint(p2.x) : from;
         top = bottom = 0;
-        pend.n = 0;
-        busy = walking = true;
+        waiting = kNone;
+        busy = true;
+        advance();
     };
     for (;;) {
         if (!drained) {
@@ -611,7 +605,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
                 base = __shfl_sync(active, base, leader);
                 const uint32_t i = base + (uint32_t)__popc(active & ((1u << lane_id()) - 1u));
                 if (i >= n) drained = true;
-                else start(i, 0, true);
+                else start(i, kNone);
             }
         }
         {
@@ -619,60 +613,55 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
             if (__ballot_sync(act, drained)) {
                 const uint32_t idle = __ballot_sync(act, drained && !busy);
                 if (idle == act) break;
-                const bool donor = walking && top > bottom;
+                const bool donor = busy && top > bottom;
                 const uint32_t donors = __ballot_sync(act, donor);
                 if (idle && donors) {
                     const Steal st = steal_round(act, idle, donors, drained && !busy, donor, stack, bottom, top);
                     const uint32_t from_idx = __shfl_sync(act, idx, st.from >= 0 ? st.from : (int)lane_id());
-                    if (st.from >= 0) start(from_idx, st.subtree, false);
+                    if (st.from >= 0) start(from_idx, st.subtree);
                 }
             }
         }
 #pragma unroll
-        for (uint32_t sub = 0; sub < kStepsPerTurn; sub++) if (walking && pend.can_step()) {
-            // one inner step of the any-hit walk (mesh_tracer.h:51-114); hit leaves wait
-            float ln, rn, lf, rf;
-            float4 la, lb, xa, xb;
-            load_node(nodes, left, la, lb);
-            load_node(nodes, left + 1, xa, xb);
-            bump<COUNT>(w.mesh_nodes, 2);
-            bool hl = hit_node(r, la, lb, ln, lf) && ln < aux;
-            bool hr = hit_node(r, xa, xb, rn, rf) && rn < aux;
-            uint32_t lc = node_first(lb), rc = node_first(xb);
-            uint32_t lcount = node_leaf_count(lb), rcount = node_leaf_count(xb);
-            if (hl && lcount) pend.push(lc, lcount, lf);
-            if (hr && rcount) pend.push(rc, rcount, rf);
-            bool go_left = hl && !lcount, go_right = hr && !rcount;
-            if (go_left) {
-                if (go_right) {
-                    if (!push_entry(stack, bottom, top, rc)) { err |= kErrStack; walking = false; }
-                }
-                left = lc;
-            } else if (go_right) {
-                left = rc;
-            } else if (top == bottom) {
-                walking = false;
-                top = bottom = 0;
-            } else {
-                left = stack[--top];
+        for (uint32_t sub = 0; sub < kStepsPerTurn; sub++) {
+            if (busy && !(next & kWideLeaf)) {
+                // One node of the any-hit walk: the hit child that reaches
+                // furthest is next (a shadow ray's occluder is rarely the
+                // surface it starts on), the others go on the stack.
+                uint4 child;
+                float t0[4], t1[4];
+                const uint32_t hits = wide_hits(S.wide_nodes, next, r, wr, aux, child, t0, t1);
+                bump<COUNT>(w.mesh_nodes, 4);
+                next = kNone;
+                float reach = -1.0f;
+                const uint32_t c[4] = {child.x, child.y, child.z, child.w};
+#pragma unroll
+                for (int s = 0; s < 4; s++)
+                    if (hits >> s & 1u) {
+                        const bool further = t1[s] > reach;
+                        const uint32_t other = further ? next : c[s];
+                        next = further ? c[s] : next;
+                        reach = further ? t1[s] : reach;
+                        if (other != kNone) stack[top++] = other;
+                    }
+                advance();
             }
         }
-        if (leaf_round(pend.n > 0, walking && pend.can_step()) && pend.n) {
-            Hit h;
-            h.distance = aux;
-            bool hit = hit_triangles<COUNT>(S.tri_hot, tri_offset + pend.first0, pend.count0, pend.clip0, r, h,
-                                            true, w);
-            pend.pop();
-            if (hit) {
+        if (leaf_round(waiting != kNone, busy && !(next & kWideLeaf)) && waiting != kNone) {
+            const float4 *leaf = S.wide_leaves + 8 * (size_t)(waiting & ~kWideLeaf);
+            float4 a, b;
+            load_node(leaf, 0, a, b);
+            float ln, lf;
+            waiting = kNone;
+            if (wide_leaf_box(r, wr, a, b, ln, lf) && ln < aux && any_triangle<COUNT>(S, leaf, tri_offset, b, minr(lf, aux), r, w)) {
                 atomicOr(A.masks + (tag >> 6), 1ull << (tag & 63u));
-                walking = false;
+                next = kNone;
                 top = bottom = 0;
-                pend.n = 0;
             }
+            advance();
         }
-        if (busy && !walking && pend.n == 0) busy = false;
+        if (busy && next == kNone && waiting == kNone && top == bottom) busy = false;
     }
-    if (err) atomicOr(F.error_flags, err);
     flush_stage<COUNT>(A.counters, w);
 }
 
@@ -689,15 +678,23 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
 //                  every geometry it visits (k), tests implicit primitives on
 //                  the spot (culling by the best implicit hit so far) and
 //                  appends one candidate per reached mesh instance;
-//   extend_mesh    a persistent kernel: every lane takes one mesh-BVH step
-//                  per loop turn in the reference's order and fetches the
-//                  next candidate when its walk ends; finished candidates
+//   extend_mesh    a persistent kernel: every lane walks one candidate at a
+//                  time over the four-wide BVH, nearest child first, and
+//                  fetches the next when its walk ends; finished candidates
 //                  publish (distance, k) with a 64-bit atomicMin per ray;
 //   extend_resolve the candidate whose (distance, k) is the ray's minimum
 //                  writes the hit record.
 // Cross-candidate culling keeps ties (<=), so the winner is the reference's.
+// Within a mesh the walk visits leaves in another order than the reference,
+// which keeps the first of two hits at the same distance and skips a leaf
+// whose box begins at or beyond the current hit.  A hit beyond its own box's
+// near distance is reached whatever was hit before, so the nearest hit is the
+// reference's unless another lies between it and its box's near distance
+// (rounding can put the near distance behind the hit) or at the same
+// distance: such a ray is traced whole (k_extend_overflow; none of the 2.07 M
+// primary rays of the 1080p mesh frame).
 // Candidate records (4 float4): (local origin, clip) (local direction, slot)
-// (node offset, triangle offset, first child, 0) (geometry, mesh, k, found);
+// (wide root, triangle offset, plane bound, 0) (geometry, mesh, k, found);
 // a finished walk overwrites the third with (t, u, v, triangle | behind << 31)
 // and sets `found`.  The ray keys live in the shadow-mask array, which is
 // free until the shadow stage.
@@ -705,6 +702,8 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
 SLIM_D unsigned long long hit_key(float t, uint32_t k) {
     return ((unsigned long long)__float_as_uint(t) << 32) | k;
 }
+// Boxes up to this factor beyond the best hit are still entered.
+constexpr float kReachSlack = 1.0f + 0x1p-18f;
 // No hit yet: distance +inf (the culling bound reads the high word as a float).
 constexpr unsigned long long kNoHitKey = (0x7F800000ull << 32) | 0xFFFFFFFFull;
 
@@ -777,13 +776,13 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
                     }
                     continue;
                 }
-                uint32_t q = warp_append(A.pair_count, true);
-                if (q >= cap) { full = true; continue; }
+                const bool wide = m.wide_root != kNoWideBVH;
+                uint32_t q = warp_append(A.pair_count, wide);
+                if (!wide || q >= cap) { full = true; continue; }
                 float4 *p = A.pairs + 4 * (size_t)q;
                 p[0] = make_float4(local.o.x, local.o.y, local.o.z, clip);
                 p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(slot));
-                p[2] = make_float4(__uint_as_float(m.node_offset), __uint_as_float(m.tri_offset),
-                                   __uint_as_float(node_first(rb)), 0.0f);
+                p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
                 p[3] = make_float4(__uint_as_float(gi), __uint_as_float(g.mesh), __uint_as_float(k), 0.0f);
             }
         };
@@ -844,7 +843,8 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
     flush_stage<COUNT>(A.counters, w);
 }
 
-// Rays whose candidates did not fit: the reference's whole closest-hit walk.
+// Rays whose candidates did not fit, or whose mesh walk left the nearest hit
+// undecided: the reference's whole closest-hit walk.
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(256) k_extend_overflow(DevScene S0, DevFrame F0, QueueArgs A) {
     const uint32_t n = A.pair_count[2];
@@ -872,17 +872,30 @@ template <bool COUNT>
 __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_mesh(DevScene S, DevFrame F, QueueArgs A) {
     const uint32_t cap = A.pair_capacity * 3u / 4u;
     const uint32_t n = *A.pair_count < cap ? *A.pair_count : cap;
-    uint32_t stack[kStackCapacity];
-    uint32_t err = 0;
+    uint2 stack[kStackCapacity];    // (node or leaf, its near distance)
     Work w = {};
-    bool busy = false, walking = false;
-    uint32_t idx = 0, slot = 0, left = 0, top = 0, tri_offset = 0, tri = 0, k = 0;
-    const float4 *nodes = nullptr;
-    float lc = 0.0f, bu = 0.0f, bv = 0.0f;
-    bool found = false, behind = false;
+    bool busy = false;
+    uint32_t idx = 0, slot = 0, top = 0, tri_offset = 0, tri = 0, k = 0;
+    uint32_t next = kNone, waiting = kNone;
+    float lc = 0.0f, lc_near = 0.0f, reach = 0.0f, bu = 0.0f, bv = 0.0f;
+    bool found = false, behind = false, unsure = false;
     Ray r;
-    PendingLeaves pend;
-    pend.n = 0;
+    WideRay wr;
+    // the nearest waiting entry that can still hold a closer hit
+    auto pop = [&]() -> uint32_t {
+        while (top) {
+            const uint2 e = stack[--top];
+            if (__uint_as_float(e.y) <= reach) return e.x;
+        }
+        return kNone;
+    };
+    auto advance = [&]() {          // as in k_shadow_mesh
+        if (next == kNone) next = pop();
+        if (next != kNone && (next & kWideLeaf) && waiting == kNone) {
+            waiting = next;
+            next = pop();
+        }
+    };
     for (;;) {
         const bool fetch = fetch_round(!busy);
         if (!busy && fetch) {
@@ -896,77 +909,88 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
             const float4 *p = A.pairs + 4 * (size_t)idx;
             float4 p0 = p[0], p1 = p[1], p2 = p[2];
             reset(r, xyz(p0), xyz(p1));
+            wr = wide_setup(r, p2.z);
             lc = p0.w;
             slot = __float_as_uint(p1.w);
             k = __float_as_uint(p[3].z);
-            nodes = S.mesh_nodes + 2 * (size_t)__float_as_uint(p2.x);
+            reach = fminf(lc, __uint_as_float((uint32_t)(A.masks[slot] >> 32))) * kReachSlack;
+            next = __float_as_uint(p2.x);
+            waiting = kNone;
             tri_offset = __float_as_uint(p2.y);
-            left = __float_as_uint(p2.z);
             top = 0;
-            found = false;
-            pend.n = 0;
-            busy = walking = true;
+            found = unsure = false;
+            busy = true;
         }
 #pragma unroll
-        for (uint32_t sub = 0; sub < kStepsPerTurn; sub++) if (walking && pend.can_step()) {
-            // one inner step of MeshTracer::trace (mesh_tracer.h:51-114); hit leaves
-            // wait and are tested in the order the walk reached them
-            const float gb = __uint_as_float((uint32_t)(A.masks[slot] >> 32));
-            float ln, rn, lf, rf;
-            float4 la, lb, xa, xb;
-            load_node(nodes, left, la, lb);
-            load_node(nodes, left + 1, xa, xb);
-            bump<COUNT>(w.mesh_nodes, 2);
-            bool hl = hit_node(r, la, lb, ln, lf) && ln < lc && ln <= gb;
-            bool hr = hit_node(r, xa, xb, rn, rf) && rn < lc && rn <= gb;
-            uint32_t lchild = node_first(lb), rchild = node_first(xb);
-            uint32_t lcount = node_leaf_count(lb), rcount = node_leaf_count(xb);
-            if (hl && lcount) pend.push(lchild, lcount, lf);
-            if (hr && rcount) pend.push(rchild, rcount, rf);
-            bool go_left = hl && !lcount, go_right = hr && !rcount;
-            if (go_left) {
-                if (go_right) {
-                    if (ln > rn) { uint32_t t = lchild; lchild = rchild; rchild = t; }
-                    if (top >= (uint32_t)kStackCapacity) { err |= kErrStack; walking = false; }
-                    else stack[top++] = rchild;
+        for (uint32_t sub = 0; sub < kStepsPerTurn; sub++) if (busy && !(next & kWideLeaf)) {
+            uint4 child;
+            float t0[4], t1[4];
+            const uint32_t hits = wide_hits(S.wide_nodes, next, r, wr, reach, child, t0, t1);
+            bump<COUNT>(w.mesh_nodes, 4);
+            // the nearest hit child is next, the others go on the stack
+            float near = INFINITY;
+            next = kNone;
+            const uint32_t c[4] = {child.x, child.y, child.z, child.w};
+#pragma unroll
+            for (int s = 0; s < 4; s++)
+                if (hits >> s & 1u) {
+                    const bool nearer = t0[s] < near;
+                    const uint32_t other = nearer ? next : c[s];
+                    const float far = nearer ? near : t0[s];
+                    next = nearer ? c[s] : next;
+                    near = nearer ? t0[s] : near;
+                    if (other != kNone) stack[top++] = make_uint2(other, __float_as_uint(far));
                 }
-                left = lchild;
-            } else if (go_right) {
-                left = rchild;
-            } else if (top == 0) {
-                walking = false;
-            } else {
-                left = stack[--top];
-            }
+            advance();
         }
-        if (leaf_round(pend.n > 0, walking && pend.can_step()) && pend.n) {
+        if (leaf_round(waiting != kNone, busy && !(next & kWideLeaf)) && waiting != kNone) {
             // MeshTracer::hitTriangles (mesh_tracer.h:23-49) with the leaf's far clip
-            const float gb = __uint_as_float((uint32_t)(A.masks[slot] >> 32));
-            float closest = minr(pend.clip0, lc);
-            for (uint32_t i = 0; i < pend.count0; i++) {
-                bump<COUNT>(w.triangles);
-                const uint32_t t_index = pend.first0 + i;
-                const float4 *t4 = S.tri_hot + 3 * (size_t)(tri_offset + t_index);
-                float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
-                float3 pp = xyz(a), nn = f3(a.w, b.x, b.y);
-                float tt; float3 pos; bool bh;
-                if (!hit_plane(r, pp, nn, tt, pos, bh)) continue;
-                float3 q = pos - pp;
-                float ux = b.z * q.x + c.x * q.y + c.z * q.z;
-                float uy = b.w * q.x + c.y * q.y + c.w * q.z;
-                if (ux < 0 || uy < 0 || (ux + uy) > 1 || tt >= closest || tt > gb) continue;
-                closest = tt;
-                lc = tt;
-                bu = ux;
-                bv = uy;
-                behind = bh;
-                tri = t_index;
-                found = true;
+            const float4 *leaf = S.wide_leaves + 8 * (size_t)(waiting & ~kWideLeaf);
+            float4 na, nb;
+            load_node(leaf, 0, na, nb);
+            float ln, lf;
+            waiting = kNone;
+            if (wide_leaf_box(r, wr, na, nb, ln, lf)) {
+                const float gb = __uint_as_float((uint32_t)(A.masks[slot] >> 32));
+                const uint32_t count = node_leaf_count(nb), first = node_first(nb);
+                for (uint32_t i = 0; i < count; i++) {
+                    bump<COUNT>(w.triangles);
+                    const float4 *t4 = leaf_triangle(S, leaf, tri_offset + first, i);
+                    float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
+                    float3 pp = xyz(a), nn = f3(a.w, b.x, b.y);
+                    float tt; float3 pos; bool bh;
+                    if (!hit_plane(r, pp, nn, tt, pos, bh)) continue;
+                    float3 q = pos - pp;
+                    float ux = b.z * q.x + c.x * q.y + c.z * q.z;
+                    float uy = b.w * q.x + c.y * q.y + c.w * q.z;
+                    if (ux < 0 || uy < 0 || (ux + uy) > 1 || tt >= lf || tt > gb) continue;
+                    if (tt >= lc) {
+                        unsure |= found && tt <= lc_near;
+                        continue;
+                    }
+                    unsure |= found && lc <= ln;
+                    lc = tt;
+                    lc_near = maxr(ln, tt);
+                    bu = ux;
+                    bv = uy;
+                    behind = bh;
+                    tri = first + i;
+                    found = true;
+                }
+                reach = fminf(lc, gb) * kReachSlack;
             }
-            pend.pop();
+            advance();
         }
-        if (busy && !walking && pend.n == 0) {
+        if (busy && next == kNone && waiting == kNone && !top) {
             float4 *p = A.pairs + 4 * (size_t)idx;
+            if (unsure) {
+                // two hits so close together that the order of the visits
+                // decides between them: the ray is traced whole, once, in
+                // the reference's order (k_extend_overflow)
+                if (atomicMin(A.masks + slot, 0ull))
+                    reinterpret_cast<uint32_t *>(A.shadow_rays)[atomicAdd(A.pair_count + 2, 1u)] = slot;
+                found = false;
+            }
             if (found) {
                 p[2] = make_float4(lc, bu, bv, __uint_as_float(tri | ((uint32_t)behind << 31)));
                 atomicMin(A.masks + slot, hit_key(lc, k));
@@ -975,7 +999,6 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
             busy = false;
         }
     }
-    if (err) atomicOr(F.error_flags, err);
     flush_stage<COUNT>(A.counters, w);
 }
 

@@ -1,0 +1,143 @@
+// Collapse of a binary mesh BVH to the four-wide form (see wide_bvh.h).
+#include "wide_bvh.h"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+namespace slim {
+
+namespace {
+
+void box_of(const SlimBVHNode &n, float lo[3], float hi[3]) {
+    lo[0] = n.aabb.min.x; lo[1] = n.aabb.min.y; lo[2] = n.aabb.min.z;
+    hi[0] = n.aabb.max.x; hi[1] = n.aabb.max.y; hi[2] = n.aabb.max.z;
+}
+
+bool boxes_nest(const SlimBVHNode *nodes, uint32_t count) {
+    for (uint32_t i = 0; i < count; i++) {
+        float lo[3], hi[3];
+        box_of(nodes[i], lo, hi);
+        for (int a = 0; a < 3; a++)
+            if (!(std::fabs(lo[a]) < 1e18f && std::fabs(hi[a]) < 1e18f)) return false;
+        if (nodes[i].leaf_count) continue;
+        for (uint32_t c = nodes[i].first_index; c < nodes[i].first_index + 2; c++) {
+            float clo[3], chi[3];
+            box_of(nodes[c], clo, chi);
+            for (int a = 0; a < 3; a++)
+                if (!(clo[a] >= lo[a] && chi[a] <= hi[a])) return false;
+        }
+    }
+    return true;
+}
+
+float from_bits(uint32_t u) {
+    float f;
+    memcpy(&f, &u, 4);
+    return f;
+}
+uint32_t to_bits(float f) {
+    uint32_t u;
+    memcpy(&u, &f, 4);
+    return u;
+}
+
+// The 16 bits of a plane at offset x >= 0, its float's lower half being
+// `below`: the largest that decodes to x or less, or the smallest that
+// decodes to x or more.  (Offset 0 with bits below reads as a denormal,
+// which the walk's margin covers.)
+uint32_t plane_bits(double x, bool up, uint32_t below) {
+    uint32_t h = to_bits((float)x) >> 16;
+    if (up) {
+        while (h && (double)from_bits((h - 1) << 16 | below) >= x) h--;
+        while ((double)from_bits(h << 16 | below) < x) h++;
+    } else {
+        while ((double)from_bits((h + 1) << 16 | below) <= x) h++;
+        while (h && (double)from_bits(h << 16 | below) > x) h--;
+    }
+    return h;
+}
+
+double surface(const SlimBVHNode &n) {
+    const double x = (double)n.aabb.max.x - n.aabb.min.x, y = (double)n.aabb.max.y - n.aabb.min.y,
+                 z = (double)n.aabb.max.z - n.aabb.min.z;
+    return x * y + y * z + z * x;
+}
+
+}  // namespace
+
+float wide_offset(const uint32_t words[2], int s) {
+    return from_bits(s & 1 ? words[s >> 1] : words[s >> 1] << 16);
+}
+
+uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const float *hot, uint32_t stack,
+                        std::vector<WideNode> &out, std::vector<WideLeaf> &leaves, float &extent) {
+    if (!node_count || nodes[0].leaf_count || !boxes_nest(nodes, node_count)) return kNoWideBVH;
+    const size_t root = out.size(), first_leaf = leaves.size();
+    std::vector<uint32_t> source{0};       // binary node of every wide node from `root` on
+    std::vector<uint32_t> waiting{0};      // nodes a walk may have waiting when it enters it
+    for (size_t w = 0; w < source.size(); w++) {
+        // open the largest inner child until four are reached
+        uint32_t child[4] = {nodes[source[w]].first_index, nodes[source[w]].first_index + 1};
+        uint32_t count = 2;
+        while (count < 4) {
+            int open = -1;
+            for (uint32_t k = 0; k < count; k++)
+                if (!nodes[child[k]].leaf_count && (open < 0 || surface(nodes[child[k]]) > surface(nodes[child[open]])))
+                    open = (int)k;
+            if (open < 0) break;
+            const uint32_t first = nodes[child[open]].first_index;
+            child[open] = first;
+            child[count++] = first + 1;
+        }
+        WideNode n{};
+        float far_corner[3];
+        box_of(nodes[source[w]], n.origin, far_corner);
+        for (uint32_t k = 0; k < 4; k++) {
+            uint32_t lo_bits[3], hi_bits[3];
+            n.child[k] = kWideLeaf;
+            for (int a = 0; a < 3; a++) {
+                lo_bits[a] = to_bits(1e30f) >> 16;
+                hi_bits[a] = to_bits(-1e30f) >> 16;
+            }
+            if (k < count) {
+                const SlimBVHNode &c = nodes[child[k]];
+                float lo[3], hi[3];
+                box_of(c, lo, hi);
+                for (int a = 0; a < 3; a++) {
+                    lo_bits[a] = plane_bits((double)lo[a] - n.origin[a], false, k & 1 ? n.lo[a][k >> 1] : 0u);
+                    hi_bits[a] = plane_bits((double)hi[a] - n.origin[a], true, k & 1 ? n.hi[a][k >> 1] : 0u);
+                }
+                if (c.leaf_count) {
+                    n.child[k] = kWideLeaf | (uint32_t)leaves.size();
+                    WideLeaf leaf{};
+                    leaf.node = c;
+                    for (uint32_t t = 0; t < c.leaf_count && t < 2; t++)
+                        memcpy(leaf.triangles[t], hot + 12 * (size_t)(c.first_index + t), sizeof(leaf.triangles[t]));
+                    leaves.push_back(leaf);
+                } else {
+                    n.child[k] = (uint32_t)(root + source.size());
+                    source.push_back(child[k]);
+                    waiting.push_back(waiting[w] + count - 1);
+                }
+            }
+            for (int a = 0; a < 3; a++) {
+                n.lo[a][k >> 1] |= lo_bits[a] << (16 * (k & 1));
+                n.hi[a][k >> 1] |= hi_bits[a] << (16 * (k & 1));
+            }
+        }
+        out.push_back(n);
+        if (waiting[w] + count - 1 > stack || leaves.size() >= kWideLeaf || root + source.size() >= kWideLeaf) {
+            out.resize(root);
+            leaves.resize(first_leaf);
+            return kNoWideBVH;
+        }
+    }
+    float lo[3], hi[3], largest = 0.0f;
+    box_of(nodes[0], lo, hi);
+    for (int a = 0; a < 3; a++) largest = std::max({largest, std::fabs(lo[a]), std::fabs(hi[a])});
+    extent = 1.05f * largest + 1e-12f;     // a rounded offset is at most 2^-7 of itself, hence of 2 largest, further out
+    return (uint32_t)root;
+}
+
+}  // namespace slim
