@@ -457,17 +457,45 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
 // against 1.29 ms.
 constexpr uint32_t kStepsPerTurn = 2;
 
-// Warp-uniform decision: should idle lanes take new candidates now?  Idle
-// lanes wait until a third of the warp is idle (or nobody is busy) and
-// then fetch together, so the fetch code -- one atomic, the candidate loads,
-// the ray set-up -- runs for several lanes at once instead of for the one or
-// two that finished this turn (config 2: 1.94 -> 1.82 ms).
-constexpr uint32_t kFetchFraction = 3;   // fetch when idle lanes >= active lanes / kFetchFraction
-SLIM_D bool fetch_round(bool idle) {
-    const uint32_t act = __activemask();
-    const uint32_t idle_mask = __ballot_sync(act, idle);
-    return idle_mask && (kFetchFraction * (uint32_t)__popc(idle_mask) >= (uint32_t)__popc(act) || idle_mask == act);
-}
+// A warp's view of the candidate queue; uniform over the warp.  Idle lanes
+// wait until a third of the warp is idle and then fetch together, so the
+// fetch code -- one atomic, the candidate loads, the ray set-up -- runs for
+// several lanes at once (a third 1.287, a quarter 1.291, a sixth 1.300 ms).
+// A launch with few candidates spreads them over its warps, and idle lanes
+// take over subtrees of their warp's walks: from the start of such a launch,
+// at the end of a large one.
+constexpr uint32_t kFetchFraction = 3;
+// Candidates per warp below which a launch is such a one: at 8 the frame with
+// 8 bounces takes 2.39 ms, at 16 the same, the light meshes at 637 x 359 0.67
+// and 0.69 ms (not sharing: 2.53 and 0.70).
+constexpr uint32_t kSparse = 8;
+struct Feed {
+    uint32_t n, quota;
+    bool drained;
+    SLIM_D Feed(uint32_t n_) : n(n_), drained(n_ == 0) {
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        quota = min(32u, (n + warps - 1) / warps);
+    }
+    SLIM_D bool sparse() const { return quota < kSparse; }
+    // lanes with a subtree to give, where idle lanes may take one
+    SLIM_D uint32_t donors(bool donor) const {
+        return drained || sparse() ? __ballot_sync(0xFFFFFFFFu, donor) : 0u;
+    }
+    SLIM_D bool fetch(uint32_t idle, uint32_t donors) const {
+        if (drained) return false;
+        return sparse() ? !donors && __popc(idle) >= 24 : kFetchFraction * (uint32_t)__popc(idle) >= 32u;
+    }
+    // Candidate of this lane (n: none) when the `idle` lanes fetch.
+    SLIM_D uint32_t take(uint32_t *cursor, uint32_t idle) {
+        const uint32_t lanes = min((uint32_t)__popc(idle), quota);
+        uint32_t base = 0;
+        if (lane_id() == 0) base = atomicAdd(cursor, lanes);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        drained = base + lanes >= n;
+        const uint32_t rank = (uint32_t)__popc(idle & ((1u << lane_id()) - 1u));
+        return (idle >> lane_id() & 1u) && rank < lanes ? min(base + rank, n) : n;
+    }
+};
 
 // No node: as a reference it counts as a leaf, so no lane steps into it.
 constexpr uint32_t kNone = 0xFFFFFFFFu;
@@ -482,6 +510,11 @@ SLIM_D bool leaf_round(bool waiting, bool can_step) {
     const uint32_t step_mask = __ballot_sync(act, can_step);
     return wait_mask && (kLeafFraction * (uint32_t)__popc(wait_mask) >= (uint32_t)__popc(act) || !step_mask);
 }
+SLIM_D bool fetch_round(bool idle) {
+    const uint32_t act = __activemask();
+    const uint32_t idle_mask = __ballot_sync(act, idle);
+    return idle_mask && (kFetchFraction * (uint32_t)__popc(idle_mask) >= (uint32_t)__popc(act) || idle_mask == act);
+}
 
 // 128-thread blocks, capped at 64 registers for the any-hit walks (32 warps
 // per SM) and 72 for the closest-hit walks (28): 1.284 ms; any hit at 9 or
@@ -495,36 +528,36 @@ constexpr int kMeshBlock = 128;
 #define SLIM_EXTEND_MESH_BLOCKS 7
 #endif
 
-// Drain phase of the persistent any-hit kernel.  Once the pair queue is
-// empty, a lane with nothing left to walk takes the deepest pending subtree
-// (the bottom entry of the stack) of a lane of its warp that is still
-// walking, so the last long walks of a launch spread over the warp instead
-// of running one lane each while the rest of the warp waits.  The i-th idle
-// lane (in lane order) takes from the i-th lane with a pending subtree; the
-// giver removes the entry from its stack.  Exact: an any-hit result is the
-// OR over the leaves a walk reaches, whatever the order (1.46 -> 1.45 ms;
-// with 8 bounces, whose late rounds are almost all tail, 3.00 -> 2.91 ms).
+// Sharing of walks: an idle lane takes the deepest waiting subtree (the
+// bottom entry of the stack) of a lane of its warp that is still walking, so
+// the last walks of a launch, and the few walks of a small one, spread over
+// their warps instead of running one lane each.  The i-th idle lane (in lane
+// order) takes from the i-th lane with a waiting subtree; the giver removes
+// the entry from its stack.
 struct Steal {
-    int from;           // giving lane for a taker, else -1
-    uint32_t subtree;   // stack entry handed over (valid for a taker)
+    int from;                   // giving lane for a taker, else -1
+    bool gave;
+    uint32_t subtree, near;     // stack entry handed over (valid for a taker)
 };
-SLIM_D Steal steal_round(uint32_t act, uint32_t idle_mask, uint32_t donor_mask, bool idle, bool donor,
-                         uint32_t *stack, uint32_t &bottom, uint32_t &top) {
+template <typename Entry>
+SLIM_D Steal steal_round(uint32_t idle_mask, uint32_t donor_mask, const Entry *stack, uint32_t &bottom, uint32_t &top) {
     const uint32_t below = (1u << lane_id()) - 1u;
     const uint32_t pairs = min((uint32_t)__popc(idle_mask), (uint32_t)__popc(donor_mask));
     const uint32_t my_idle_rank = (uint32_t)__popc(idle_mask & below);
-    const bool taker = idle && my_idle_rank < pairs;
-    const bool giver = donor && (uint32_t)__popc(donor_mask & below) < pairs;
-    uint32_t give = 0;
-    if (giver) {
-        give = stack[bottom++];
-        if (bottom == top) bottom = top = 0;
+    const bool taker = (idle_mask >> lane_id() & 1u) && my_idle_rank < pairs;
+    Steal st;
+    st.gave = (donor_mask >> lane_id() & 1u) && (uint32_t)__popc(donor_mask & below) < pairs;
+    uint2 give = make_uint2(0, 0);
+    if (st.gave) {
+        if constexpr (sizeof(Entry) == sizeof(uint2)) give = stack[bottom];
+        else give.x = stack[bottom];
+        if (++bottom == top) bottom = top = 0;
     }
     uint32_t m = donor_mask;
     for (uint32_t j = 0; taker && j < my_idle_rank; j++) m &= m - 1u;
-    const int src = taker ? __ffs(m) - 1 : (int)lane_id();
-    Steal st;
-    st.subtree = __shfl_sync(act, give, src);
+    const int src = taker ? __ffs((int)m) - 1 : (int)lane_id();
+    st.subtree = __shfl_sync(0xFFFFFFFFu, give.x, src);
+    st.near = sizeof(Entry) == sizeof(uint2) ? __shfl_sync(0xFFFFFFFFu, give.y, src) : 0u;
     st.from = taker ? src : -1;
     return st;
 }
@@ -558,10 +591,10 @@ SLIM_D bool any_triangle(const DevScene &S, const float4 *leaf, uint32_t tri_off
 
 template <bool COUNT>
 __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_mesh(DevScene S, DevFrame F, QueueArgs A) {
-    const uint32_t n = *A.pair_count < A.pair_capacity ? *A.pair_count : A.pair_capacity;
+    Feed feed(min(*A.pair_count, A.pair_capacity));
     uint32_t stack[kStackCapacity];
     Work w = {};
-    bool busy = false, drained = false;
+    bool busy = false;
     uint32_t idx = 0, tag = 0, top = 0, bottom = 0, tri_offset = 0;
     uint32_t next = kNone;          // node or leaf the walk goes to
     uint32_t waiting = kNone;       // a leaf to be tested
@@ -595,31 +628,18 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
         advance();
     };
     for (;;) {
-        if (!drained) {
-            const bool fetch = fetch_round(!busy);
-            if (!busy && fetch) {
-                uint32_t active = __activemask();
-                int leader = __ffs(active) - 1;
-                uint32_t base = 0;
-                if ((int)lane_id() == leader) base = atomicAdd(A.pair_cursor, (uint32_t)__popc(active));
-                base = __shfl_sync(active, base, leader);
-                const uint32_t i = base + (uint32_t)__popc(active & ((1u << lane_id()) - 1u));
-                if (i >= n) drained = true;
-                else start(i, kNone);
-            }
-        }
-        {
-            const uint32_t act = __activemask();
-            if (__ballot_sync(act, drained)) {
-                const uint32_t idle = __ballot_sync(act, drained && !busy);
-                if (idle == act) break;
-                const bool donor = busy && top > bottom;
-                const uint32_t donors = __ballot_sync(act, donor);
-                if (idle && donors) {
-                    const Steal st = steal_round(act, idle, donors, drained && !busy, donor, stack, bottom, top);
-                    const uint32_t from_idx = __shfl_sync(act, idx, st.from >= 0 ? st.from : (int)lane_id());
-                    if (st.from >= 0) start(from_idx, st.subtree);
-                }
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
+        if (idle) {
+            const uint32_t donors = feed.donors(busy && top > bottom);
+            if (feed.fetch(idle, donors)) {
+                const uint32_t i = feed.take(A.pair_cursor, idle);
+                if (i < feed.n) start(i, kNone);
+            } else if (donors) {
+                const Steal st = steal_round(idle, donors, stack, bottom, top);
+                const uint32_t from_idx = __shfl_sync(0xFFFFFFFFu, idx, st.from >= 0 ? st.from : (int)lane_id());
+                if (st.from >= 0) start(from_idx, st.subtree);
+            } else if (feed.drained && idle == 0xFFFFFFFFu) {
+                break;
             }
         }
 #pragma unroll
@@ -693,10 +713,15 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
 // (rounding can put the near distance behind the hit) or at the same
 // distance: such a ray is traced whole (k_extend_overflow; none of the 2.07 M
 // primary rays of the 1080p mesh frame).
+// Few walks are shared like the any-hit ones (a loop of its own, without the
+// sharing's cost for large launches, whose ends the other rays' walks cover):
+// a part culls by the ray's published distance and, if its hit is still the ray's nearest when it ends, appends a
+// record of its own; parts with hits at the same distance, or with a hit that
+// is not beyond its box's near distance, leave the ray undecided.
 // Candidate records (4 float4): (local origin, clip) (local direction, slot)
-// (wide root, triangle offset, plane bound, 0) (geometry, mesh, k, found);
-// a finished walk overwrites the third with (t, u, v, triangle | behind << 31)
-// and sets `found`.  The ray keys live in the shadow-mask array, which is
+// (wide root, triangle offset, plane bound, 0) (geometry, mesh, k, found); a
+// walk that ends with the ray's nearest hit so far overwrites the third with
+// (t, u, v, triangle | behind << 31) and sets `found`.  The ray keys live in the shadow-mask array, which is
 // free until the shadow stage.
 
 SLIM_D unsigned long long hit_key(float t, uint32_t k) {
@@ -868,22 +893,21 @@ __global__ void __launch_bounds__(256) k_extend_overflow(DevScene S0, DevFrame F
     flush_stage<COUNT>(A.counters, w);
 }
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_mesh(DevScene S, DevFrame F, QueueArgs A) {
-    const uint32_t cap = A.pair_capacity * 3u / 4u;
-    const uint32_t n = *A.pair_count < cap ? *A.pair_count : cap;
+template <bool COUNT, bool SHARE>
+SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint32_t cap) {
     uint2 stack[kStackCapacity];    // (node or leaf, its near distance)
     Work w = {};
     bool busy = false;
-    uint32_t idx = 0, slot = 0, top = 0, tri_offset = 0, tri = 0, k = 0;
+    uint32_t idx = 0, slot = 0, top = 0, bottom = 0, tri_offset = 0, tri = 0, k = 0;
     uint32_t next = kNone, waiting = kNone;
     float lc = 0.0f, lc_near = 0.0f, reach = 0.0f, bu = 0.0f, bv = 0.0f;
     bool found = false, behind = false, unsure = false;
+    bool piece = false, shared = false;     // part of another lane's walk; a walk that gave parts away
     Ray r;
     WideRay wr;
     // the nearest waiting entry that can still hold a closer hit
     auto pop = [&]() -> uint32_t {
-        while (top) {
+        while (top > bottom) {
             const uint2 e = stack[--top];
             if (__uint_as_float(e.y) <= reach) return e.x;
         }
@@ -896,30 +920,69 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
             next = pop();
         }
     };
+    // the ray's other candidates and, of a shared walk, its other parts cull by
+    // the published distance; two parts with the same leave the ray undecided
+    auto publish = [&]() { unsure |= atomicMin(A.masks + slot, hit_key(lc, k)) == hit_key(lc, k); };
+    // candidate i from its root, or from a node of its walk
+    auto start = [&](uint32_t i, uint32_t from) {
+        const float4 *p = A.pairs + 4 * (size_t)i;
+        const float4 p0 = p[0], p1 = p[1], p3 = p[3];
+        float4 p2 = p[2];
+        piece = shared = SHARE && from != kNone;
+        if (piece) {        // the walk's own result may have taken the place of its mesh
+            const DevMesh &m = S.meshes[__float_as_uint(p3.y)];
+            p2 = make_float4(__uint_as_float(from), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
+        }
+        idx = i;
+        reset(r, xyz(p0), xyz(p1));
+        wr = wide_setup(r, p2.z);
+        lc = p0.w;
+        slot = __float_as_uint(p1.w);
+        k = __float_as_uint(p3.z);
+        reach = fminf(lc, __uint_as_float((uint32_t)(A.masks[slot] >> 32))) * kReachSlack;
+        next = __float_as_uint(p2.x);
+        waiting = kNone;
+        tri_offset = __float_as_uint(p2.y);
+        top = bottom = 0;
+        found = unsure = false;
+        busy = true;
+        advance();
+    };
     for (;;) {
-        const bool fetch = fetch_round(!busy);
-        if (!busy && fetch) {
-            uint32_t active = __activemask();
-            int leader = __ffs(active) - 1;
-            uint32_t base = 0;
-            if ((int)lane_id() == leader) base = atomicAdd(A.pair_cursor, (uint32_t)__popc(active));
-            base = __shfl_sync(active, base, leader);
-            idx = base + (uint32_t)__popc(active & ((1u << lane_id()) - 1u));
-            if (idx >= n) break;
-            const float4 *p = A.pairs + 4 * (size_t)idx;
-            float4 p0 = p[0], p1 = p[1], p2 = p[2];
-            reset(r, xyz(p0), xyz(p1));
-            wr = wide_setup(r, p2.z);
-            lc = p0.w;
-            slot = __float_as_uint(p1.w);
-            k = __float_as_uint(p[3].z);
-            reach = fminf(lc, __uint_as_float((uint32_t)(A.masks[slot] >> 32))) * kReachSlack;
-            next = __float_as_uint(p2.x);
-            waiting = kNone;
-            tri_offset = __float_as_uint(p2.y);
-            top = 0;
-            found = unsure = false;
-            busy = true;
+        if constexpr (!SHARE) {
+            const bool fetch = fetch_round(!busy);
+            if (!busy && fetch) {
+                uint32_t active = __activemask();
+                int leader = __ffs(active) - 1;
+                uint32_t base = 0;
+                if ((int)lane_id() == leader) base = atomicAdd(A.pair_cursor, (uint32_t)__popc(active));
+                base = __shfl_sync(active, base, leader);
+                const uint32_t i = base + (uint32_t)__popc(active & ((1u << lane_id()) - 1u));
+                if (i >= feed.n) break;
+                start(i, kNone);
+            }
+        } else {
+            const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
+            if (idle) {
+                const uint32_t donors = feed.donors(busy && top > bottom);
+                if (feed.fetch(idle, donors)) {
+                    const uint32_t i = feed.take(A.pair_cursor, idle);
+                    if (i < feed.n) start(i, kNone);
+                } else if (donors) {
+                    const Steal st = steal_round(idle, donors, stack, bottom, top);
+                    if (st.gave) {
+                        // a hit at or before its own box's near distance is sure
+                        // only against hits of the same lane
+                        unsure |= found && lc_near > lc;
+                        if (found && !shared) publish();
+                        shared = true;
+                    }
+                    const uint32_t from_idx = __shfl_sync(0xFFFFFFFFu, idx, st.from >= 0 ? st.from : (int)lane_id());
+                    if (st.from >= 0) start(from_idx, st.subtree);
+                } else if (feed.drained && idle == 0xFFFFFFFFu) {
+                    break;
+                }
+            }
         }
 #pragma unroll
         for (uint32_t sub = 0; sub < kStepsPerTurn; sub++) if (busy && !(next & kWideLeaf)) {
@@ -952,6 +1015,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
             waiting = kNone;
             if (wide_leaf_box(r, wr, na, nb, ln, lf)) {
                 const float gb = __uint_as_float((uint32_t)(A.masks[slot] >> 32));
+                const float before = lc;
                 const uint32_t count = node_leaf_count(nb), first = node_first(nb);
                 for (uint32_t i = 0; i < count; i++) {
                     bump<COUNT>(w.triangles);
@@ -968,7 +1032,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
                         unsure |= found && tt <= lc_near;
                         continue;
                     }
-                    unsure |= found && lc <= ln;
+                    unsure |= (found && lc <= ln) || (shared && tt <= ln);
                     lc = tt;
                     lc_near = maxr(ln, tt);
                     bu = ux;
@@ -977,29 +1041,55 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
                     tri = first + i;
                     found = true;
                 }
+                if (SHARE && shared && lc < before) publish();
                 reach = fminf(lc, gb) * kReachSlack;
             }
             advance();
         }
-        if (busy && next == kNone && waiting == kNone && !top) {
+        if (busy && next == kNone && waiting == kNone && top == bottom) {
             float4 *p = A.pairs + 4 * (size_t)idx;
-            if (unsure) {
-                // two hits so close together that the order of the visits
-                // decides between them: the ray is traced whole, once, in
-                // the reference's order (k_extend_overflow)
-                if (atomicMin(A.masks + slot, 0ull))
-                    reinterpret_cast<uint32_t *>(A.shadow_rays)[atomicAdd(A.pair_count + 2, 1u)] = slot;
-                found = false;
+            const float4 result = make_float4(lc, bu, bv, __uint_as_float(tri | ((uint32_t)behind << 31)));
+            if (!shared && !unsure) {
+                // publishes and waits for no answer (waiting: 225 -> 284 us for the first round's launch)
+                if (found) {
+                    p[2] = result;
+                    p[3].w = 1.0f;
+                    atomicMin(A.masks + slot, hit_key(lc, k));
+                }
+            } else {
+                const bool best = found && !unsure && __ldcg(A.masks + slot) == hit_key(lc, k);
+                uint32_t record = idx;
+                if (best && piece) {
+                    // a part's hit gets a record of its own behind the candidates
+                    record = feed.n + atomicAdd(A.pair_count + 3, 1u);
+                    unsure = record >= cap;
+                }
+                if (unsure) {
+                    // two hits so close together that the order of the visits
+                    // decides between them: the ray is traced whole, once, in
+                    // the reference's order (k_extend_overflow)
+                    if (atomicMin(A.masks + slot, 0ull))
+                        reinterpret_cast<uint32_t *>(A.shadow_rays)[atomicAdd(A.pair_count + 2, 1u)] = slot;
+                } else if (best) {
+                    float4 *o = A.pairs + 4 * (size_t)record;
+                    const float4 p1 = p[1], p3 = p[3];
+                    if (piece) o[1] = p1;
+                    o[2] = result;
+                    o[3] = make_float4(p3.x, p3.y, p3.z, 1.0f);
+                }
             }
-            if (found) {
-                p[2] = make_float4(lc, bu, bv, __uint_as_float(tri | ((uint32_t)behind << 31)));
-                atomicMin(A.masks + slot, hit_key(lc, k));
-            }
-            p[3].w = found ? 1.0f : 0.0f;
             busy = false;
         }
     }
     flush_stage<COUNT>(A.counters, w);
+}
+
+template <bool COUNT>
+__global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_mesh(DevScene S, DevFrame F, QueueArgs A) {
+    const uint32_t cap = A.pair_capacity * 3u / 4u;
+    Feed feed(min(*A.pair_count, cap));
+    if (feed.sparse()) extend_walks<COUNT, true>(S, A, feed, cap);
+    else extend_walks<COUNT, false>(S, A, feed, cap);
 }
 
 // The candidate holding its ray's minimum (distance, k) writes the hit
@@ -1007,7 +1097,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(256) k_extend_resolve(DevScene S0, DevFrame F0, QueueArgs A) {
     const uint32_t cap = A.pair_capacity * 3u / 4u;
-    const uint32_t n = *A.pair_count < cap ? *A.pair_count : cap;
+    const uint32_t n = min(min(*A.pair_count, cap) + A.pair_count[3], cap);
     Work w = {};
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
         const float4 *p = A.pairs + 4 * (size_t)idx;
@@ -1519,8 +1609,8 @@ cudaError_t trace_round(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         // the queued rays' hit records are in place already (training paths
         // that start at their cache vertex)
     } else if (L.split_extend && B.pair_capacity >= 4) {
-        // [3] candidates, [4] candidate cursor, [5] overflowed rays
-        r = cudaMemsetAsync(B.queue_count + 3, 0, 3 * sizeof(uint32_t), stream);
+        // [3] candidates, [4] candidate cursor, [5] rays traced whole, [6] records of parts of walks
+        r = cudaMemsetAsync(B.queue_count + 3, 0, 4 * sizeof(uint32_t), stream);
         if (r != cudaSuccess) return r;
         k_extend_scene<COUNT, BATCH><<<L.grid((const void *)k_extend_scene<COUNT, BATCH>, L.bound), L.block, 0, stream>>>(S, F, A);
         count_launch();
