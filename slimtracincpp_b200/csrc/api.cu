@@ -437,6 +437,25 @@ int upload_lights(Context &c, const SlimSceneData *s) {
     return SLIM_OK;
 }
 
+// The leaves of a scene BVH small enough to test one by one (see DevScene).
+void list_leaves(DevScene &S, const SlimBVHNode *nodes, uint32_t node_count) {
+    S.listed_leaves = 0;
+    if (nodes[0].leaf_count || node_count > 2 * kMaxListedLeaves + 64 || !boxes_nest(nodes, node_count)) return;
+    uint32_t count = 0;
+    std::vector<uint8_t> reached(node_count, 0);
+    reached[0] = 1;
+    for (uint32_t i = 0; i < node_count; i++) {
+        if (!reached[i]) continue;
+        if (!nodes[i].leaf_count) {
+            reached[nodes[i].first_index] = reached[nodes[i].first_index + 1] = 1;
+            continue;
+        }
+        if (count == kMaxListedLeaves || i > 255) return;
+        S.leaf_node[count++] = (uint8_t)i;
+    }
+    S.listed_leaves = count;
+}
+
 // Parent-before-child order of the scene BVH's inner nodes, reversed, so the
 // refit kernel can process it level by level bottom-up in one launch.
 void build_refit_order(Context &c, const SlimBVHNode *nodes, uint32_t node_count) {
@@ -471,6 +490,7 @@ int upload_scene_bvh(Context &c, const SlimSceneData *s) {
     c.scene.leaf_geometry = c.d_leaf_geometry.ptr;
     c.scene.scene_node_count = n;
     c.scene.flags = s->flags;
+    list_leaves(c.scene, s->bvh.nodes, n);
     return SLIM_OK;
 }
 
@@ -2205,6 +2225,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         S.light_count = s->counts.lights;
         S.scene_node_count = s->bvh.node_count;
         S.flags = s->flags;
+        list_leaves(S, s->bvh.nodes, s->bvh.node_count);
         uint32_t emissive = 0, instances = 0;
         for (uint32_t g = 0; g < s->counts.geometries; g++) {
             const SlimGeometry &G = s->geometries[g];

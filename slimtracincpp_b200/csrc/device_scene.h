@@ -73,7 +73,13 @@ struct DevScene {
     uint32_t emissive_quad_count;
     uint32_t flags;                // SLIM_SCENE_HAD_EMISSIVE_QUADS
     uint32_t scene_node_count;
+    // Leaves of a small scene BVH (node indices; count 0: larger than
+    // kMaxListedLeaves, a root leaf, or boxes that do not nest), for rays that
+    // test every leaf's box instead of walking the tree.
+    uint32_t listed_leaves;
+    uint8_t leaf_node[32];
 };
+constexpr uint32_t kMaxListedLeaves = 32;
 
 // Per-frame parameters of a render launch.
 struct DevFrame {

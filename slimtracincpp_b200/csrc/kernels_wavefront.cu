@@ -393,6 +393,16 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
         bool occluded = false;
         float ln, rn, lf, rf;
         float4 ra, rb;
+        if (!COUNT && S.listed_leaves && finite_ray(ray)) {
+            for (uint32_t leaves = leaves_hit(S, ray, Ld); leaves && !occluded; leaves &= leaves - 1u) {
+                load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], ra, rb);
+                hit_box_finite(ray, ra, rb, ln, lf);
+                occluded = shadow_leaf<COUNT>(S, A, tag, node_first(rb), node_leaf_count(rb), lf, ray, Ld, mesh_stack,
+                                              err, w);
+            }
+            if (occluded) atomicOr(A.masks + (tag >> 6), 1ull << (tag & 63u));
+            continue;
+        }
         load_node(S.scene_nodes, 0, ra, rb);
         bump<COUNT>(w.scene_nodes);
         if (hit_node(ray, ra, rb, ln, lf) && ln < Ld) {
@@ -727,8 +737,6 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
 SLIM_D unsigned long long hit_key(float t, uint32_t k) {
     return ((unsigned long long)__float_as_uint(t) << 32) | k;
 }
-// Boxes up to this factor beyond the best hit are still entered.
-constexpr float kReachSlack = 1.0f + 0x1p-18f;
 // No hit yet: distance +inf (the culling bound reads the high word as a float).
 constexpr unsigned long long kNoHitKey = (0x7F800000ull << 32) | 0xFFFFFFFFull;
 
@@ -753,64 +761,96 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
         int best_geo = -1;
         uint32_t best_k = 0, k = 0;
         bool full = false;
+        // A visible mesh instance of a leaf with near and far distances ln, lf:
+        // a candidate, or a single-leaf mesh's triangles here.
+        auto instance = [&](uint32_t gi, const Geo &g, float ln, float lf, Nearest *seen) {
+            const float clip = lf + kEps;
+            Ray local;
+            bump<COUNT>(w.geometries);
+            localize(local, r.o, r.d, g);
+            const DevMesh &m = S.meshes[g.mesh];
+            float bn, bf;
+            if (!hit_aabb(local, m.aabb_min[0], m.aabb_min[1], m.aabb_min[2], m.aabb_max[0], m.aabb_max[1],
+                          m.aabb_max[2], bn, bf))
+                return;
+            const float4 *nodes = S.mesh_nodes + 2 * (size_t)m.node_offset;
+            float4 ra, rb;
+            float rn, rf;
+            load_node(nodes, 0, ra, rb);
+            bump<COUNT>(w.mesh_nodes);
+            // the root test with the largest distance the reference could have used
+            if (!(hit_node(local, ra, rb, rn, rf) && rn < clip && rn <= hit.distance)) return;
+            if (node_leaf_count(rb)) {
+                // a single-leaf mesh (mesh_tracer.h:66-70): its triangles here
+                Hit mh;
+                mh.distance = clip;
+                if (hit_triangles<COUNT>(S.tri_hot, m.tri_offset, m.tri_count, rf, local, mh, false, w) &&
+                    (seen ? seen->take(mh.distance, maxr(ln, rn), hit.distance) : mh.distance < hit.distance)) {
+                    mh.uv_coverage = __ldg(&S.tri_cold[4 * (size_t)(m.tri_offset + mh.id) + 3].w);
+                    best_geo = (int)gi;
+                    best_k = k;
+                    hit = mh;
+                    hit.NdotRd = -(dot(hit.normal, local.d));
+                }
+                return;
+            }
+            const bool wide = m.wide_root != kNoWideBVH;
+            uint32_t q = warp_append(A.pair_count, wide);
+            if (!wide || q >= cap) { full = true; return; }
+            float4 *p = A.pairs + 4 * (size_t)q;
+            p[0] = make_float4(local.o.x, local.o.y, local.o.z, clip);
+            p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(slot));
+            p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
+            p[3] = make_float4(__uint_as_float(gi), __uint_as_float(g.mesh), __uint_as_float(k), 0.0f);
+        };
         // one scene leaf: [first, first + count) geometries, far distance lf
         auto leaf = [&](uint32_t first, uint32_t count, float lf) {
             Hit aux;
             aux.distance = minr(lf + kEps, hit.distance);
-            const float clip = lf + kEps;
             Ray local;
             for (uint32_t i = 0; i < count; i++, k++) {
                 uint32_t gi = __ldg(S.leaf_geometry + first + i);
                 Geo g = load_geo(S, gi);
                 if (!(g.flags & SLIM_GEOMETRY_IS_VISIBLE)) continue;
-                if (g.type != SLIM_GEOMETRY_MESH) {
-                    if (hit_geometry_local<COUNT>(S, g, r, local, aux, false, nullptr, err, w) &&
-                        aux.distance < hit.distance) {
-                        best_geo = (int)gi;
-                        best_k = k;
-                        hit = aux;
-                        hit.NdotRd = -(dot(hit.normal, local.d));
-                    }
-                    continue;
+                if (g.type == SLIM_GEOMETRY_MESH) {
+                    instance(gi, g, 0.0f, lf, nullptr);
+                } else if (hit_geometry_local<COUNT>(S, g, r, local, aux, false, nullptr, err, w) &&
+                           aux.distance < hit.distance) {
+                    best_geo = (int)gi;
+                    best_k = k;
+                    hit = aux;
+                    hit.NdotRd = -(dot(hit.normal, local.d));
                 }
-                bump<COUNT>(w.geometries);
-                localize(local, r.o, r.d, g);
-                const DevMesh &m = S.meshes[g.mesh];
-                float bn, bf;
-                if (!hit_aabb(local, m.aabb_min[0], m.aabb_min[1], m.aabb_min[2], m.aabb_max[0], m.aabb_max[1],
-                              m.aabb_max[2], bn, bf))
-                    continue;
-                const float4 *nodes = S.mesh_nodes + 2 * (size_t)m.node_offset;
-                float4 ra, rb;
-                float rn, rf;
-                load_node(nodes, 0, ra, rb);
-                bump<COUNT>(w.mesh_nodes);
-                // the root test with the largest distance the reference could have used
-                if (!(hit_node(local, ra, rb, rn, rf) && rn < clip && rn <= hit.distance)) continue;
-                if (node_leaf_count(rb)) {
-                    // a single-leaf mesh (mesh_tracer.h:66-70): its triangles here
-                    Hit mh;
-                    mh.distance = clip;
-                    if (hit_triangles<COUNT>(S.tri_hot, m.tri_offset, m.tri_count, rf, local, mh, false, w) &&
-                        mh.distance < hit.distance) {
-                        mh.uv_coverage = __ldg(&S.tri_cold[4 * (size_t)(m.tri_offset + mh.id) + 3].w);
-                        best_geo = (int)gi;
-                        best_k = k;
-                        hit = mh;
-                        hit.NdotRd = -(dot(hit.normal, local.d));
-                    }
-                    continue;
-                }
-                const bool wide = m.wide_root != kNoWideBVH;
-                uint32_t q = warp_append(A.pair_count, wide);
-                if (!wide || q >= cap) { full = true; continue; }
-                float4 *p = A.pairs + 4 * (size_t)q;
-                p[0] = make_float4(local.o.x, local.o.y, local.o.z, clip);
-                p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(slot));
-                p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
-                p[3] = make_float4(__uint_as_float(gi), __uint_as_float(g.mesh), __uint_as_float(k), 0.0f);
             }
         };
+        // Small scenes: every leaf's box, then the implicit primitives of the
+        // hit ones, then their mesh instances, the best implicit hit already
+        // known.  Candidates are numbered in that order from 1; an implicit hit
+        // has 0, and a candidate at exactly the ray's best distance that is not
+        // its holder sends the ray to the whole walk (k_extend_resolve).
+        bool listed = !COUNT && S.listed_leaves && finite_ray(r);
+        if (listed) {
+            const uint32_t leaves = leaves_hit(S, r, INFINITY);
+            Nearest seen;
+            best_geo = closest_of_leaves<COUNT>(S, leaves, r, hit, seen, err, w);
+            for (uint32_t rest = leaves; rest && !seen.unsure; rest &= rest - 1u) {
+                float4 a, b;
+                float ln, lf;
+                load_node(S.scene_nodes, S.leaf_node[__ffs((int)rest) - 1], a, b);
+                hit_box_finite(r, a, b, ln, lf);
+                if (ln > hit.distance * kReachSlack) continue;
+                const uint32_t first = node_first(b), count = node_leaf_count(b);
+                for (uint32_t i = 0; i < count; i++) {
+                    const uint32_t gi = __ldg(S.leaf_geometry + first + i);
+                    const Geo g = load_geo(S, gi);
+                    if (!(g.flags & SLIM_GEOMETRY_IS_VISIBLE) || g.type != SLIM_GEOMETRY_MESH) continue;
+                    k++;
+                    instance(gi, g, ln, lf, &seen);
+                }
+            }
+            best_k = 0;
+            full |= seen.unsure;
+        } else {
         float ln, rn, lf, rf;
         float4 a, b;
         load_node(S.scene_nodes, 0, a, b);
@@ -853,8 +893,10 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
                 }
             }
         }
+        }
         if (full) {
-            // the candidate queue ran out: the ray is traced whole afterwards
+            // the candidate queue ran out, or the order of the tests decides:
+            // the ray is traced whole afterwards
             // (k_extend_overflow); key 0 matches no candidate (hit distances
             // are never 0: the plane test rejects an origin on the plane)
             A.masks[slot] = 0ull;
@@ -1105,7 +1147,13 @@ __global__ void __launch_bounds__(256) k_extend_resolve(DevScene S0, DevFrame F0
         if (p3.w == 0.0f) continue;
         const float4 p1 = p[1], p2 = p[2];
         const uint32_t slot = __float_as_uint(p1.w);
-        if (A.masks[slot] != hit_key(p2.x, __float_as_uint(p3.z))) continue;
+        const unsigned long long best = A.masks[slot];
+        if (best != hit_key(p2.x, __float_as_uint(p3.z))) {
+            // two candidates at the same distance: the order of the visits decides
+            if ((uint32_t)(best >> 32) == __float_as_uint(p2.x) && best && atomicExch(A.masks + slot, 0ull))
+                reinterpret_cast<uint32_t *>(A.shadow_rays)[atomicAdd(A.pair_count + 2, 1u)] = slot;
+            continue;
+        }
         uint32_t pid = 0;
         if (BATCH) pid = __float_as_uint(A.rays_in[2 * (size_t)slot + 1].w);
         const DevScene &S = scene_of<BATCH>(S0, A, pid);

@@ -131,6 +131,31 @@ SLIM_D bool hit_node(const Ray &r, float4 a, float4 b, float &nearD, float &farD
     return hit_aabb(r, a.x, a.y, a.z, a.w, b.x, b.y, nearD, farD);
 }
 
+SLIM_D float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+SLIM_D float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// hit_node for a ray whose distances are finite (`finite_ray`): max and min
+// then order them as the reference's comparisons do, in half the instructions.
+SLIM_D bool hit_box_finite(const Ray &r, float4 a, float4 b, float &near, float &far) {
+    const float3 lo = f3(r.nx ? a.w : a.x, r.ny ? b.x : a.y, r.nz ? b.y : a.z);
+    const float3 hi = f3(r.nx ? a.x : a.w, r.ny ? a.y : b.x, r.nz ? a.z : b.y);
+    const float3 t0 = mul_add(lo, r.rcp, r.so), t1 = mul_add(hi, r.rcp, r.so);
+    near = fmaxf(max3(t0.x, t0.y, t0.z), 0.0f);
+    far = min3(t1.x, t1.y, t1.z);
+    return near <= far;
+}
+SLIM_D bool finite_ray(const Ray &r) {
+    return max3(fabsf(r.rcp.x), fabsf(r.rcp.y), fabsf(r.rcp.z)) < 1e18f &&
+           max3(fabsf(r.so.x), fabsf(r.so.y), fabsf(r.so.z)) < 1e18f;
+}
+
 // Ray::hitsPlane (ray.h:61-82)
 SLIM_D bool hit_plane(const Ray &r, float3 p, float3 n, float &t, float3 &pos, bool &from_behind) {
     float NdotRd = dot(n, r.d);
@@ -516,6 +541,80 @@ SLIM_D int hit_geometries(const DevScene &S, uint32_t first, uint32_t count, flo
     return hit_geo;
 }
 
+// The leaves of a small scene whose boxes the ray hits before `reach`: bit j
+// is leaf S.leaf_node[j].  A leaf's box lies in the boxes above it, so the
+// tree walk reaches the same leaves; the loop has no stack, no waiting loads
+// and no divergence.
+SLIM_D uint32_t leaves_hit(const DevScene &S, const Ray &r, float reach) {
+    uint32_t hit = 0;
+#pragma unroll 4
+    for (uint32_t j = 0; j < S.listed_leaves; j++) {
+        float4 a, b;
+        float near, far;
+        load_node(S.scene_nodes, S.leaf_node[j], a, b);
+        if (hit_box_finite(r, a, b, near, far) && near < reach) hit |= 1u << j;
+    }
+    return hit;
+}
+// Boxes up to this factor beyond the best hit are still looked into.
+constexpr float kReachSlack = 1.0f + 0x1p-18f;
+
+// What a closest hit has seen so far when geometries are tested in another
+// order than the reference's.  The reference keeps the first of two hits at
+// the same distance and skips a leaf whose box begins at or beyond the
+// current hit; a hit beyond its own leaf's near distance is reached whatever
+// was hit before.  So the nearest hit is the reference's unless another one
+// lies at the same distance or between it and its leaf's near distance
+// (rounding can put that behind the hit): then the order decides.
+struct Nearest {
+    float near = 0.0f;      // no hit from here up to `near` was taken
+    bool unsure = false;
+    // How far hits are looked for, given the best distance.
+    SLIM_D float reach(float best) const { return maxr(best, near); }
+    // A hit at t in a leaf with near distance `ln`: is it the new nearest?
+    SLIM_D bool take(float t, float ln, float best) {
+        const bool found = near > 0.0f;
+        if (t < best) {
+            unsure |= found && best <= ln;
+            near = maxr(t, ln);
+            return true;
+        }
+        unsure |= found && t <= near;
+        return false;
+    }
+};
+
+// scene_trace over the listed leaves, closest hit of implicit primitives.
+template <bool COUNT>
+SLIM_D int closest_of_leaves(const DevScene &S, uint32_t leaves, const Ray &r, Hit &hit, Nearest &seen, uint32_t &err,
+                             Work &w) {
+    int best = -1;
+    while (leaves) {
+        float4 a, b;
+        float ln, lf;
+        load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], a, b);
+        leaves &= leaves - 1u;
+        hit_box_finite(r, a, b, ln, lf);
+        if (ln > hit.distance * kReachSlack) continue;
+        const uint32_t first = node_first(b), count = node_leaf_count(b);
+        Hit aux;
+        for (uint32_t i = 0; i < count; i++) {
+            const uint32_t gi = __ldg(S.leaf_geometry + first + i);
+            const Geo g = load_geo(S, gi);
+            if (!(g.flags & SLIM_GEOMETRY_IS_VISIBLE) || g.type == SLIM_GEOMETRY_MESH) continue;
+            Ray local;
+            aux.distance = minr(lf + kEps, seen.reach(hit.distance) * kReachSlack);
+            if (hit_geometry_local<COUNT>(S, g, r, local, aux, false, nullptr, err, w) &&
+                seen.take(aux.distance, ln, hit.distance)) {
+                best = (int)gi;
+                hit = aux;
+                hit.NdotRd = -(dot(hit.normal, local.d));
+            }
+        }
+    }
+    return best;
+}
+
 // SceneTracer::trace (scene_tracer.h:26-98): offsets the origin by
 // TRACE_OFFSET along the direction, then walks the scene BVH near child
 // first (both children tested per step, the far one pushed).
@@ -524,6 +623,25 @@ SLIM_D int scene_trace(const DevScene &S, Ray &r, Hit &hit, bool any_hit, float 
                        uint32_t *stack, uint32_t *mesh_stack, uint32_t &err, Work &w) {
     reset(r, scale_add(r.d, kTraceOffset, r.o), r.d);
     hit.distance = max_distance;
+    if (!COUNT && S.listed_leaves && (any_hit || !S.mesh_count) && finite_ray(r)) {
+        uint32_t leaves = leaves_hit(S, r, max_distance);
+        if (any_hit) {
+            while (leaves) {
+                float4 a, b;
+                float ln, lf;
+                load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], a, b);
+                leaves &= leaves - 1u;
+                hit_box_finite(r, a, b, ln, lf);
+                const int g = hit_geometries<COUNT>(S, node_first(b), node_leaf_count(b), lf, r, hit, true, mesh_stack, err, w);
+                if (g >= 0) return g;
+            }
+            return -1;
+        }
+        Nearest seen;
+        const int g = closest_of_leaves<COUNT>(S, leaves, r, hit, seen, err, w);
+        if (!seen.unsure) return g;
+        hit.distance = max_distance;
+    }
     float ln, rn, lf, rf;
     float4 a, b;
     load_node(S.scene_nodes, 0, a, b);

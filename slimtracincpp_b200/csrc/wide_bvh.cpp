@@ -14,23 +14,6 @@ void box_of(const SlimBVHNode &n, float lo[3], float hi[3]) {
     hi[0] = n.aabb.max.x; hi[1] = n.aabb.max.y; hi[2] = n.aabb.max.z;
 }
 
-bool boxes_nest(const SlimBVHNode *nodes, uint32_t count) {
-    for (uint32_t i = 0; i < count; i++) {
-        float lo[3], hi[3];
-        box_of(nodes[i], lo, hi);
-        for (int a = 0; a < 3; a++)
-            if (!(std::fabs(lo[a]) < 1e18f && std::fabs(hi[a]) < 1e18f)) return false;
-        if (nodes[i].leaf_count) continue;
-        for (uint32_t c = nodes[i].first_index; c < nodes[i].first_index + 2; c++) {
-            float clo[3], chi[3];
-            box_of(nodes[c], clo, chi);
-            for (int a = 0; a < 3; a++)
-                if (!(clo[a] >= lo[a] && chi[a] <= hi[a])) return false;
-        }
-    }
-    return true;
-}
-
 float from_bits(uint32_t u) {
     float f;
     memcpy(&f, &u, 4);
@@ -65,6 +48,23 @@ double surface(const SlimBVHNode &n) {
 }
 
 }  // namespace
+
+bool boxes_nest(const SlimBVHNode *nodes, uint32_t count) {
+    for (uint32_t i = 0; i < count; i++) {
+        float lo[3], hi[3];
+        box_of(nodes[i], lo, hi);
+        for (int a = 0; a < 3; a++)
+            if (!(std::fabs(lo[a]) < 1e18f && std::fabs(hi[a]) < 1e18f)) return false;
+        if (nodes[i].leaf_count) continue;
+        for (uint32_t c = nodes[i].first_index; c < nodes[i].first_index + 2; c++) {
+            float clo[3], chi[3];
+            box_of(nodes[c], clo, chi);
+            for (int a = 0; a < 3; a++)
+                if (!(clo[a] >= lo[a] && chi[a] <= hi[a])) return false;
+        }
+    }
+    return true;
+}
 
 float wide_offset(const uint32_t words[2], int s) {
     return from_bits(s & 1 ? words[s >> 1] : words[s >> 1] << 16);

@@ -6,16 +6,6 @@
 namespace slim {
 namespace dev {
 
-SLIM_D float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-SLIM_D float min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
 // A ray as the wide walk takes it: the reciprocal direction, and -o * rcp
 // with the margin for the planes a ray meets first and last.  The exact test
 // rounds plane * rcp + so once; here so -+ margin, origin * rcp + that and
@@ -78,15 +68,7 @@ SLIM_D uint32_t wide_hits(const uint4 *nodes, uint32_t i, const Ray &r, const Wi
 
 // The exact test of a leaf's box.
 SLIM_D bool wide_leaf_box(const Ray &r, const WideRay &w, float4 a, float4 b, float &near, float &far) {
-    if (!w.parallel) {
-        // finite distances: max and min order them as the reference's comparisons do
-        const float3 lo = f3(r.nx ? a.w : a.x, r.ny ? b.x : a.y, r.nz ? b.y : a.z);
-        const float3 hi = f3(r.nx ? a.x : a.w, r.ny ? a.y : b.x, r.nz ? a.z : b.y);
-        const float3 t0 = mul_add(lo, r.rcp, r.so), t1 = mul_add(hi, r.rcp, r.so);
-        near = fmaxf(max3(t0.x, t0.y, t0.z), 0.0f);
-        far = min3(t1.x, t1.y, t1.z);
-        return near <= far;
-    }
+    if (!w.parallel) return hit_box_finite(r, a, b, near, far);
     Ray exact;
     reset(exact, r.o, r.d);
     return hit_node(exact, a, b, near, far);

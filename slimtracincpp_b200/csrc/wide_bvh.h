@@ -50,4 +50,8 @@ float wide_offset(const uint32_t words[2], int s);
 uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const float *hot, uint32_t stack,
                         std::vector<WideNode> &out, std::vector<WideLeaf> &leaves, float &extent);
 
+// Every box finite (within 1e18) and inside its parent's: a slab test that
+// passes for a node then passes for everything above it.
+bool boxes_nest(const SlimBVHNode *nodes, uint32_t count);
+
 }  // namespace slim
