@@ -158,6 +158,8 @@ SlimRenderOptions initial_options() {
     return o;
 }
 
+struct LeafRange { uint32_t first, end; };
+
 struct Context {
     bool initialized = false;
     int device = -1;
@@ -177,7 +179,7 @@ struct Context {
     DevArray<WideNode> d_wide_nodes;
     DevArray<WideLeaf> d_wide_leaves;
     DevArray<SlimMaterial> d_materials;
-    DevArray<SlimLight> d_lights;
+    DevArray<float4> d_lights;
     DevArray<uint32_t> d_leaf_geometry, d_emissive_quads, d_refit_order;
     DevArray<DevMesh> d_meshes;
     DevArray<DevTexture> d_textures;
@@ -188,6 +190,8 @@ struct Context {
     DevArray<uint32_t> d_error;
     DevArray<unsigned long long> d_counters;
     std::vector<uint32_t> refit_order;
+    std::vector<LeafRange> leaf_ranges;   // of the listed scene leaves, and the geometries they name
+    std::vector<uint32_t> leaf_geometry;
     uint32_t scene_node_count = 0;
 
     DevScene scene{};
@@ -393,6 +397,40 @@ int upload_emissive(Context &c) {
     return SLIM_OK;
 }
 
+// The leaves of a scene BVH small enough to test one by one (see DevScene),
+// and [first, end) of the leaf geometry indices for each.
+void list_leaves(DevScene &S, const SlimBVHNode *nodes, uint32_t node_count, std::vector<LeafRange> &ranges) {
+    S.listed_leaves = 0;
+    ranges.clear();
+    if (nodes[0].leaf_count || node_count > 2 * kMaxListedLeaves + 64 || !boxes_nest(nodes, node_count)) return;
+    std::vector<uint8_t> reached(node_count, 0);
+    reached[0] = 1;
+    for (uint32_t i = 0; i < node_count; i++) {
+        if (!reached[i]) continue;
+        if (!nodes[i].leaf_count) {
+            reached[nodes[i].first_index] = reached[nodes[i].first_index + 1] = 1;
+            continue;
+        }
+        if (ranges.size() == kMaxListedLeaves || i > 255) {
+            ranges.clear();
+            return;
+        }
+        S.leaf_node[ranges.size()] = (uint8_t)i;
+        ranges.push_back({nodes[i].first_index, nodes[i].first_index + nodes[i].leaf_count});
+    }
+    S.listed_leaves = (uint32_t)ranges.size();
+}
+void sort_leaves(DevScene &S, const std::vector<LeafRange> &ranges, const uint32_t *leaf_geometry,
+                 const SlimGeometry *geometries) {
+    S.implicit_leaves = S.mesh_leaves = S.shadow_leaves = 0;
+    for (uint32_t j = 0; j < ranges.size(); j++)
+        for (uint32_t k = ranges[j].first; k < ranges[j].end; k++) {
+            const SlimGeometry &g = geometries[leaf_geometry[k]];
+            if (g.flags & SLIM_GEOMETRY_IS_VISIBLE) (g.type == SLIM_GEOMETRY_MESH ? S.mesh_leaves : S.implicit_leaves) |= 1u << j;
+            if (g.flags & SLIM_GEOMETRY_IS_SHADOWING) S.shadow_leaves |= 1u << j;
+        }
+}
+
 int upload_geometries(Context &c, const SlimSceneData *s) {
     uint32_t n = c.counts.geometries;
     for (uint32_t g = 0; g < n; g++) {
@@ -408,6 +446,7 @@ int upload_geometries(Context &c, const SlimSceneData *s) {
     SLIM_CUDA(cudaMemcpy(c.d_geometries.ptr, packed.data(), packed.size() * sizeof(float4), cudaMemcpyHostToDevice),
               "upload geometries");
     c.scene.geometries = c.d_geometries.ptr;
+    if (c.leaf_geometry.size() == n) sort_leaves(c.scene, c.leaf_ranges, c.leaf_geometry.data(), c.geometries.data());
     return upload_emissive(c);
 }
 
@@ -427,33 +466,27 @@ int upload_materials(Context &c, const SlimSceneData *s) {
     return c.geometries.empty() ? SLIM_OK : upload_emissive(c);
 }
 
+// Light record; the two quotients are what the glow divides out per ray
+// (core/ray.h:317-319), IEEE on both sides.
+void pack_light(const SlimLight &l, std::vector<float4> &out) {
+    const uint32_t flags = l.flags;
+    float f;
+    memcpy(&f, &flags, 4);
+    out.push_back(make_float4(l.position_or_direction.x, l.position_or_direction.y, l.position_or_direction.z, l.intensity));
+    out.push_back(make_float4(l.color[0], l.color[1], l.color[2], f));
+    out.push_back(make_float4(64.0f / l.intensity, l.intensity * (1.0f / 64.0f), 0.0f, 0.0f));
+}
+
 int upload_lights(Context &c, const SlimSceneData *s) {
     uint32_t n = c.counts.lights;
-    int rc = c.d_lights.reserve(n ? n : 1, "alloc lights");
+    int rc = c.d_lights.reserve(n ? 3 * (size_t)n : 1, "alloc lights");
     if (rc) return rc;
-    if (n) SLIM_CUDA(cudaMemcpy(c.d_lights.ptr, s->lights, n * sizeof(SlimLight), cudaMemcpyHostToDevice), "upload lights");
+    std::vector<float4> packed;
+    for (uint32_t i = 0; i < n; i++) pack_light(s->lights[i], packed);
+    if (n) SLIM_CUDA(cudaMemcpy(c.d_lights.ptr, packed.data(), packed.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload lights");
     c.scene.lights = c.d_lights.ptr;
     c.scene.light_count = n;
     return SLIM_OK;
-}
-
-// The leaves of a scene BVH small enough to test one by one (see DevScene).
-void list_leaves(DevScene &S, const SlimBVHNode *nodes, uint32_t node_count) {
-    S.listed_leaves = 0;
-    if (nodes[0].leaf_count || node_count > 2 * kMaxListedLeaves + 64 || !boxes_nest(nodes, node_count)) return;
-    uint32_t count = 0;
-    std::vector<uint8_t> reached(node_count, 0);
-    reached[0] = 1;
-    for (uint32_t i = 0; i < node_count; i++) {
-        if (!reached[i]) continue;
-        if (!nodes[i].leaf_count) {
-            reached[nodes[i].first_index] = reached[nodes[i].first_index + 1] = 1;
-            continue;
-        }
-        if (count == kMaxListedLeaves || i > 255) return;
-        S.leaf_node[count++] = (uint8_t)i;
-    }
-    S.listed_leaves = count;
 }
 
 // Parent-before-child order of the scene BVH's inner nodes, reversed, so the
@@ -490,7 +523,9 @@ int upload_scene_bvh(Context &c, const SlimSceneData *s) {
     c.scene.leaf_geometry = c.d_leaf_geometry.ptr;
     c.scene.scene_node_count = n;
     c.scene.flags = s->flags;
-    list_leaves(c.scene, s->bvh.nodes, n);
+    list_leaves(c.scene, s->bvh.nodes, n, c.leaf_ranges);
+    c.leaf_geometry.assign(s->bvh_leaf_geometry_indices, s->bvh_leaf_geometry_indices + c.counts.geometries);
+    sort_leaves(c.scene, c.leaf_ranges, c.leaf_geometry.data(), c.geometries.data());
     return SLIM_OK;
 }
 
@@ -1222,6 +1257,8 @@ int slimInitDataOnGPU(const SlimSceneData *scene) {
     c.counts = scene->counts;
     c.geometries.clear();
     c.materials.clear();
+    c.leaf_geometry.clear();
+    c.leaf_ranges.clear();
     if ((rc = upload_materials(c, scene))) return rc;
     if ((rc = upload_meshes(c, scene))) return rc;
     if ((rc = upload_textures(c, scene))) return rc;
@@ -1882,7 +1919,7 @@ struct BatchState {
     std::vector<DevFrame> h_frames;
     DevArray<float4> geometries, scene_nodes;
     DevArray<SlimMaterial> materials;
-    DevArray<SlimLight> lights;
+    DevArray<float4> lights;
     DevArray<uint32_t> leaf_geometry, emissive;
     DevArray<DevScene> scenes;
     DevArray<DevFrame> frames;
@@ -2192,7 +2229,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
     int rc;
     if ((rc = b.geometries.reserve(4 * n_geo, "alloc batch geometries"))) return rc;
     if ((rc = b.materials.reserve(n_mat, "alloc batch materials"))) return rc;
-    if ((rc = b.lights.reserve(n_light ? n_light : 1, "alloc batch lights"))) return rc;
+    if ((rc = b.lights.reserve(n_light ? 3 * n_light : 1, "alloc batch lights"))) return rc;
     if ((rc = b.scene_nodes.reserve(2 * n_node, "alloc batch scene BVHs"))) return rc;
     if ((rc = b.leaf_geometry.reserve(n_geo, "alloc batch leaf indices"))) return rc;
     if ((rc = b.emissive.reserve(n_geo, "alloc batch emissive lists"))) return rc;
@@ -2200,11 +2237,11 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
     if ((rc = b.frames.reserve(count, "alloc batch frame table"))) return rc;
     std::vector<float4> geo(4 * n_geo);
     std::vector<SlimMaterial> mat;
-    std::vector<SlimLight> lig;
+    std::vector<float4> lig;
     std::vector<SlimBVHNode> nodes;
     std::vector<uint32_t> leaf, emis;
     mat.reserve(n_mat);
-    lig.reserve(n_light);
+    lig.reserve(3 * n_light);
     nodes.reserve(n_node);
     leaf.reserve(n_geo);
     emis.reserve(n_geo);
@@ -2225,7 +2262,9 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         S.light_count = s->counts.lights;
         S.scene_node_count = s->bvh.node_count;
         S.flags = s->flags;
-        list_leaves(S, s->bvh.nodes, s->bvh.node_count);
+        std::vector<LeafRange> ranges;
+        list_leaves(S, s->bvh.nodes, s->bvh.node_count, ranges);
+        sort_leaves(S, ranges, s->bvh_leaf_geometry_indices, s->geometries);
         uint32_t emissive = 0, instances = 0;
         for (uint32_t g = 0; g < s->counts.geometries; g++) {
             const SlimGeometry &G = s->geometries[g];
@@ -2239,7 +2278,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         S.emissive_quad_count = emissive;
         og += s->counts.geometries;
         mat.insert(mat.end(), s->materials, s->materials + s->counts.materials);
-        if (s->counts.lights) lig.insert(lig.end(), s->lights, s->lights + s->counts.lights);
+        for (uint32_t l = 0; l < s->counts.lights; l++) pack_light(s->lights[l], lig);
         nodes.insert(nodes.end(), s->bvh.nodes, s->bvh.nodes + s->bvh.node_count);
         leaf.insert(leaf.end(), s->bvh_leaf_geometry_indices, s->bvh_leaf_geometry_indices + s->counts.geometries);
         b.h_scenes[r] = S;
@@ -2266,7 +2305,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
     SLIM_CUDA(cudaMemcpy(b.geometries.ptr, geo.data(), geo.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload batch geometries");
     SLIM_CUDA(cudaMemcpy(b.materials.ptr, mat.data(), mat.size() * sizeof(SlimMaterial), cudaMemcpyHostToDevice), "upload batch materials");
     if (!lig.empty())
-        SLIM_CUDA(cudaMemcpy(b.lights.ptr, lig.data(), lig.size() * sizeof(SlimLight), cudaMemcpyHostToDevice), "upload batch lights");
+        SLIM_CUDA(cudaMemcpy(b.lights.ptr, lig.data(), lig.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload batch lights");
     SLIM_CUDA(cudaMemcpy(b.scene_nodes.ptr, nodes.data(), nodes.size() * sizeof(SlimBVHNode), cudaMemcpyHostToDevice), "upload batch BVHs");
     SLIM_CUDA(cudaMemcpy(b.leaf_geometry.ptr, leaf.data(), leaf.size() * 4, cudaMemcpyHostToDevice), "upload batch leaf indices");
     if (!emis.empty())

@@ -5,6 +5,7 @@
 //   geometry       4 x float4   rotation quat | position,type | scale,material | 1/scale,flags+mesh
 //   BVH node       2 x float4   the reference's 32-byte BVHNode bytes unchanged
 //                               (min.xyz, max.x | max.yz, first_index, leaf_count/depth/flags)
+//   light          3 x float4   position or direction, intensity | colour, flags | 64/intensity, intensity/64
 //   wide node      5 x uint4    four children's boxes, for the persistent mesh walks (wide_bvh.h)
 //   wide leaf      8 x float4   a leaf's BVH node and the hot bytes of its first two triangles
 //   triangle hot   3 x float4   position, normal and the two rows of local_to_tangent
@@ -56,7 +57,7 @@ struct DevTexture {
 struct DevScene {
     const float4 *geometries;      // 4 float4 per geometry
     const SlimMaterial *materials;
-    const SlimLight *lights;
+    const float4 *lights;          // 3 float4 per light
     const float4 *scene_nodes;     // 2 float4 per node
     const uint32_t *leaf_geometry; // bvh_leaf_geometry_indices
     const DevMesh *meshes;
@@ -77,6 +78,9 @@ struct DevScene {
     // kMaxListedLeaves, a root leaf, or boxes that do not nest), for rays that
     // test every leaf's box instead of walking the tree.
     uint32_t listed_leaves;
+    // of them, those with a visible implicit primitive, a visible mesh
+    // instance, anything that casts shadows
+    uint32_t implicit_leaves, mesh_leaves, shadow_leaves;
     uint8_t leaf_node[32];
 };
 constexpr uint32_t kMaxListedLeaves = 32;

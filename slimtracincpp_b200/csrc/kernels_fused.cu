@@ -43,7 +43,7 @@ SLIM_D void render_sample(const DevScene &S, const DevFrame &F, int x, int y, ui
         if (g >= 0) {
             Geo geo = load_geo(S, (uint32_t)g);
             Mat m = load_mat(S, geo.material);
-            prepare_for_shading<COUNT>(S, geo, m, ray, hit, scaling, s, w);
+            prepare_for_shading<COUNT>(S, geo, m, ray, hit, scaling, s, w, true);
             depth = depth_at(P, hit.position);
             switch (st.render_mode) {
                 case SLIM_RENDER_UVS: color = f3(hit.u, hit.v, 1.0f); break;

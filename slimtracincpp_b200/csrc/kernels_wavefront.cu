@@ -159,20 +159,20 @@ template <bool BATCH> SLIM_D const DevFrame &frame_of(const DevFrame &F, const Q
     else return F;
 }
 
-SLIM_D void primary_ray(const DevFrame &F, uint32_t i, float3 &o, float3 &d) {
-    int x = (int)(i % F.width), y = (int)(i / F.width);
+SLIM_D void primary_ray(const DevFrame &F, uint32_t x, uint32_t y, float3 &o, float3 &d) {
     const SlimCameraRayProjection &P = F.projection;
     o = f3(P.camera_position.x, P.camera_position.y, P.camera_position.z);
-    d = normalized(primary_direction(P, x, y));
+    d = normalized(primary_direction(P, (int)x, (int)y));
 }
 
 
 SLIM_D void load_ray(const DevFrame &F, const QueueArgs &A, uint32_t slot, float3 &o, float3 &d, uint32_t &path,
                      uint32_t &pid) {
     if (!A.rays_in) {
+        const uint2 p = xy_of_slot(F.width, F.rows, slot);
         path = slot;
-        pid = F.row_begin * F.width + pixel_of_slot(F.width, F.rows, slot);
-        primary_ray(F, pid, o, d);
+        pid = (F.row_begin + p.y) * F.width + p.x;
+        primary_ray(F, p.x, F.row_begin + p.y, o, d);
         return;
     }
     float4 a = A.rays_in[2 * (size_t)slot], b = A.rays_in[2 * (size_t)slot + 1];
@@ -182,15 +182,15 @@ SLIM_D void load_ray(const DevFrame &F, const QueueArgs &A, uint32_t slot, float
     pid = __float_as_uint(b.w);
 }
 template <bool BATCH> SLIM_D float cone_scaling(const DevFrame &F, uint32_t pid) {
-    uint32_t p = pix_of<BATCH>(pid);
-    return F.cones_per_pixel ? pixel_scaling(F.projection, (int)(p % F.width), (int)(p / F.width)) : 0.0f;
+    if (!F.cones_per_pixel) return 0.0f;
+    const uint32_t p = pix_of<BATCH>(pid);
+    return pixel_scaling(F.projection, (int)(p % F.width), (int)(p / F.width));
 }
 template <bool BATCH>
 SLIM_D void write_pixel(const DevFrame &F, uint32_t pid, float3 color, float depth, bool with_depth = true) {
-    uint32_t p = pix_of<BATCH>(pid);
-    float3 c = f3(tone_mapped_baked(color.x), tone_mapped_baked(color.y), tone_mapped_baked(color.z));
-    if (with_depth) set_pixel(F, (int)(p % F.width), (int)(p / F.width), c, depth);
-    else set_pixel_color(F, (int)(p % F.width), (int)(p / F.width), c);
+    const uint32_t offset = canvas_offset_of(F, pix_of<BATCH>(pid));
+    set_color_at(F, offset, f3(tone_mapped_baked(color.x), tone_mapped_baked(color.y), tone_mapped_baked(color.z)));
+    if (with_depth) set_depth_at(F, offset, depth);
 }
 
 SLIM_D uint32_t queue_size(const QueueArgs &A) { return A.count_in ? *A.count_in : A.samples; }
@@ -243,18 +243,20 @@ __global__ void __launch_bounds__(256) k_shadow_gen(DevScene S0, DevFrame F0, Qu
         bool shaded = false;
         uint32_t lights = 0, pid = 0;
         if (live) {
-            float3 o, d;
-            uint32_t path;
-            load_ray(F0, A, slot, o, d, path, pid);
-            const DevScene &S = scene_of<BATCH>(S0, A, pid);
-            const DevFrame &F = frame_of<BATCH>(F0, A, pid);
-            lights = S.light_count;
+            // a miss reads its 16-byte record and no ray
             Hit hit;
-            int g = load_hit(A.hits, A.hit_stride, slot, hit);
-            if (g >= 0 && !at_cache_vertex<BATCH>(F, A)) {
+            const int g = load_hit(A.hits, A.hit_stride, slot, hit);
+            if (g >= 0) {
+                float3 o, d;
+                uint32_t path;
+                load_ray(F0, A, slot, o, d, path, pid);
+                const DevScene &S = scene_of<BATCH>(S0, A, pid);
+                const DevFrame &F = frame_of<BATCH>(F0, A, pid);
+                lights = S.light_count;
                 Geo geo = load_geo(S, (uint32_t)g);
                 Mat m = load_mat(S, geo.material);
-                if (!((m.flags & SLIM_MATERIAL_IS_EMISSIVE) && geo.type == SLIM_GEOMETRY_QUAD && !hit.from_behind)) {
+                if (!at_cache_vertex<BATCH>(F, A) &&
+                    !((m.flags & SLIM_MATERIAL_IS_EMISSIVE) && geo.type == SLIM_GEOMETRY_QUAD && !hit.from_behind)) {
                     Ray ray;
                     reset(ray, scale_add(d, kTraceOffset, o), d);
                     prepare_for_shading<COUNT>(S, geo, m, ray, hit, cone_scaling<BATCH>(F, pid), s, w);
@@ -264,10 +266,12 @@ __global__ void __launch_bounds__(256) k_shadow_gen(DevScene S0, DevFrame F0, Qu
                 }
             }
             if (!BATCH && A.early_depth && A.light_begin == 0) {
-                uint32_t p = pix_of<BATCH>(pid);
-                set_depth(F, (int)(p % F.width), (int)(p / F.width), shaded ? depth_at(F.projection, hit.position) : INFINITY);
+                const uint2 p = xy_of_slot(F0.width, F0.rows, slot);
+                set_depth_at(F0, canvas_offset_of(F0, (F0.row_begin + p.y) * F0.width + p.x),
+                             shaded ? depth_at(F0.projection, hit.position) : INFINITY);
             }
         }
+        if (!__any_sync(__activemask(), shaded)) continue;      // nothing to light in this warp
         for (uint32_t li = A.light_begin; li < A.light_end; li++) {
             bool want = false;
             if (shaded && li < lights) {
@@ -394,7 +398,7 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
         float ln, rn, lf, rf;
         float4 ra, rb;
         if (!COUNT && S.listed_leaves && finite_ray(ray)) {
-            for (uint32_t leaves = leaves_hit(S, ray, Ld); leaves && !occluded; leaves &= leaves - 1u) {
+            for (uint32_t leaves = leaves_hit(S, ray, Ld, S.shadow_leaves); leaves && !occluded; leaves &= leaves - 1u) {
                 load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], ra, rb);
                 hit_box_finite(ray, ra, rb, ln, lf);
                 occluded = shadow_leaf<COUNT>(S, A, tag, node_first(rb), node_leaf_count(rb), lf, ray, Ld, mesh_stack,
@@ -830,10 +834,10 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
         // its holder sends the ray to the whole walk (k_extend_resolve).
         bool listed = !COUNT && S.listed_leaves && finite_ray(r);
         if (listed) {
-            const uint32_t leaves = leaves_hit(S, r, INFINITY);
+            const uint32_t leaves = leaves_hit(S, r, INFINITY, S.implicit_leaves | S.mesh_leaves);
             Nearest seen;
-            best_geo = closest_of_leaves<COUNT>(S, leaves, r, hit, seen, err, w);
-            for (uint32_t rest = leaves; rest && !seen.unsure; rest &= rest - 1u) {
+            best_geo = closest_of_leaves<COUNT>(S, leaves & S.implicit_leaves, r, hit, seen, err, w);
+            for (uint32_t rest = leaves & S.mesh_leaves; rest && !seen.unsure; rest &= rest - 1u) {
                 float4 a, b;
                 float ln, lf;
                 load_node(S.scene_nodes, S.leaf_node[__ffs((int)rest) - 1], a, b);
@@ -1561,9 +1565,10 @@ __global__ void k_batch_generate(QueueArgs A, const uint4 *__restrict__ tiles, u
         }
         uint4 t = tiles[lo];
         const DevFrame &F = A.frames[t.x];
-        uint32_t pixel = pixel_of_slot(F.width, F.height, t.y + (s - t.w));
+        const uint2 xy = xy_of_slot(F.width, F.height, t.y + (s - t.w));
+        const uint32_t pixel = xy.y * F.width + xy.x;
         float3 o, d;
-        primary_ray(F, pixel, o, d);
+        primary_ray(F, xy.x, xy.y, o, d);
         rays[2 * (size_t)s] = make_float4(o.x, o.y, o.z, __uint_as_float(s));
         rays[2 * (size_t)s + 1] = make_float4(d.x, d.y, d.z, __uint_as_float((t.x << kBatchPixelBits) | pixel));
     }

@@ -541,11 +541,13 @@ SLIM_D int hit_geometries(const DevScene &S, uint32_t first, uint32_t count, flo
     return hit_geo;
 }
 
-// The leaves of a small scene whose boxes the ray hits before `reach`: bit j
-// is leaf S.leaf_node[j].  A leaf's box lies in the boxes above it, so the
+// The leaves `of` a small scene whose boxes the ray hits before `reach`: bit j
+// is leaf S.leaf_node[j].  Every box is tested: leaving out those not asked
+// for costs more in the loop than it saves (implicit scenes 95 against 89 us).
+// A leaf's box lies in the boxes above it, so the
 // tree walk reaches the same leaves; the loop has no stack, no waiting loads
 // and no divergence.
-SLIM_D uint32_t leaves_hit(const DevScene &S, const Ray &r, float reach) {
+SLIM_D uint32_t leaves_hit(const DevScene &S, const Ray &r, float reach, uint32_t of) {
     uint32_t hit = 0;
 #pragma unroll 4
     for (uint32_t j = 0; j < S.listed_leaves; j++) {
@@ -554,7 +556,7 @@ SLIM_D uint32_t leaves_hit(const DevScene &S, const Ray &r, float reach) {
         load_node(S.scene_nodes, S.leaf_node[j], a, b);
         if (hit_box_finite(r, a, b, near, far) && near < reach) hit |= 1u << j;
     }
-    return hit;
+    return hit & of;
 }
 // Boxes up to this factor beyond the best hit are still looked into.
 constexpr float kReachSlack = 1.0f + 0x1p-18f;
@@ -624,7 +626,7 @@ SLIM_D int scene_trace(const DevScene &S, Ray &r, Hit &hit, bool any_hit, float 
     reset(r, scale_add(r.d, kTraceOffset, r.o), r.d);
     hit.distance = max_distance;
     if (!COUNT && S.listed_leaves && (any_hit || !S.mesh_count) && finite_ray(r)) {
-        uint32_t leaves = leaves_hit(S, r, max_distance);
+        uint32_t leaves = leaves_hit(S, r, max_distance, any_hit ? S.shadow_leaves : S.implicit_leaves);
         if (any_hit) {
             while (leaves) {
                 float4 a, b;
@@ -864,16 +866,20 @@ SLIM_D float3 sample_slot(const DevScene &S, const Mat &m, uint32_t slot, float 
 
 // SurfaceShader::prepareForShading (surface_shader.h:61-107).  `ray` is the
 // traced world-space ray (origin already offset), `hit` the local-space hit.
+// The texture footprint is left out for a material without maps (`coverage`:
+// a debug mode shows it), which nothing reads.
 template <bool COUNT>
 SLIM_D void prepare_for_shading(const DevScene &S, const Geo &g, const Mat &m, const Ray &ray, Hit &hit,
-                                float scaling, Surface &s, Work &w) {
+                                float scaling, Surface &s, Work &w, bool coverage = false) {
     hit.u *= m.rep_u;
     hit.v *= m.rep_v;
     if (hit.from_behind) hit.normal = -hit.normal;
-    float cone = hit.distance * scaling;
-    cone *= cone;
-    cone *= cone;
-    hit.uv_coverage *= cone / (m.rep_u * m.rep_v * hit.NdotRd * fabsf(dot(one_minus(hit.normal), g.s)));
+    if (coverage || m.texture_count) {
+        float cone = hit.distance * scaling;
+        cone *= cone;
+        cone *= cone;
+        hit.uv_coverage *= cone / (m.rep_u * m.rep_v * hit.NdotRd * fabsf(dot(one_minus(hit.normal), g.s)));
+    }
     hit.position = at(ray, hit.distance);
     hit.normal = normalized(qrot(g.axis, g.w, g.s * hit.normal));
     bool has_maps = m.texture_count != 0;
@@ -897,12 +903,12 @@ SLIM_D void prepare_for_shading(const DevScene &S, const Geo &g, const Mat &m, c
 
 struct LightRec { float3 color, pos; float intensity; uint32_t flags; };
 SLIM_D LightRec load_light(const DevScene &S, uint32_t i) {
-    const SlimLight *p = S.lights + i;
+    const float4 a = __ldg(S.lights + 3 * (size_t)i), b = __ldg(S.lights + 3 * (size_t)i + 1);
     LightRec l;
-    l.color = ld3(p->color);
-    l.pos = ld3(&p->position_or_direction.x);
-    l.intensity = __ldg(&p->intensity);
-    l.flags = __ldg(reinterpret_cast<const uint32_t *>(&p->flags)) & 0xFFu;
+    l.pos = xyz(a);
+    l.intensity = a.w;
+    l.color = xyz(b);
+    l.flags = __float_as_uint(b.w);
     return l;
 }
 
@@ -1005,8 +1011,8 @@ SLIM_D void add_glow(const DevScene &S, const Ray &ray, float &hit_distance, flo
     for (uint32_t i = 0; i < S.light_count; i++) {
         LightRec l = load_light(S, i);
         if (l.flags & SLIM_LIGHT_IS_DIRECTIONAL) continue;
-        float radius = l.intensity * kLightIntensityRadius;
-        float orr = kLightRadiusIntensity / l.intensity;
+        const float4 c2 = __ldg(S.lights + 3 * (size_t)i + 2);
+        const float orr = c2.x, radius = c2.y;
         float t_max = hit_distance * orr;
         float3 rc = (l.pos - ray.o) * orr;
         float b = dot(ray.d, rc);
@@ -1028,7 +1034,7 @@ SLIM_D void add_glow(const DevScene &S, const Ray &ray, float &hit_distance, flo
 
 SLIM_D float tone_mapped_baked(float c) {                                            // base.h:777-786
     float x = c - 0.004f;
-    if (x < 0.0f) x = 0.0f;
+    if (x <= 0.0f) return 0.0f;      // 0 / 0.06: a pixel that no light reached
     float x2s = x * x * 6.2f;
     return (x2s + x * 0.5f) / (x2s + x * 1.7f + 0.06f);
 }
@@ -1088,10 +1094,10 @@ SLIM_D float3 primary_direction(const SlimCameraRayProjection &p, int x, int y) 
 // rows the slots run through 8-column groups; the columns past the last
 // full group, and a last band shorter than 4 rows, keep row order.  A
 // bijection of [0, width * height); config 2: 2.08 -> 2.03 ms.
-SLIM_D uint32_t pixel_of_slot(uint32_t W, uint32_t H, uint32_t slot) {
+SLIM_D uint2 xy_of_slot(uint32_t W, uint32_t H, uint32_t slot) {
     const uint32_t band = 4u * W;
     const uint32_t b = slot / band;
-    if (b >= H / 4u) return slot;
+    if (b >= H / 4u) return make_uint2(slot % W, slot / W);
     const uint32_t j = slot - b * band;
     const uint32_t groups = W / 8u, g = j / 32u;
     uint32_t x, y;
@@ -1103,7 +1109,11 @@ SLIM_D uint32_t pixel_of_slot(uint32_t W, uint32_t H, uint32_t slot) {
         x = groups * 8u + r % rest;
         y = b * 4u + r / rest;
     }
-    return y * W + x;
+    return make_uint2(x, y);
+}
+SLIM_D uint32_t pixel_of_slot(uint32_t W, uint32_t H, uint32_t slot) {
+    const uint2 p = xy_of_slot(W, H, slot);
+    return p.y * W + p.x;
 }
 
 SLIM_D float pixel_scaling(const SlimCameraRayProjection &p, int x, int y) {
@@ -1125,13 +1135,17 @@ SLIM_D uint32_t canvas_offset(const DevFrame &F, int x, int y) {
         ? ((F.stride * (uint32_t)(y >> 1) + (uint32_t)(x >> 1)) * 4 + 2 * (uint32_t)(y & 1) + (uint32_t)(x & 1))
         : (F.stride * (uint32_t)y + (uint32_t)x);
 }
-SLIM_D void set_pixel_color(const DevFrame &F, int x, int y, float3 c) {
+// The same for sample index p = y * width + x: itself on a plain canvas
+// without padding, so most samples divide nothing.
+SLIM_D uint32_t canvas_offset_of(const DevFrame &F, uint32_t p) {
+    return F.antialias != SLIM_AA_SSAA && F.stride == F.width ? p : canvas_offset(F, (int)(p % F.width), (int)(p / F.width));
+}
+SLIM_D void set_color_at(const DevFrame &F, uint32_t offset, float3 c) {
     c = f3(clamp01(c.x), clamp01(c.y), clamp01(c.z));
     c = c * (c * 1.0f);
-    F.pixels[canvas_offset(F, x, y)] = make_float4(c.x, c.y, c.z, 1.0f);
+    F.pixels[offset] = make_float4(c.x, c.y, c.z, 1.0f);
 }
-SLIM_D void set_depth(const DevFrame &F, int x, int y, float depth) {
-    uint32_t offset = canvas_offset(F, x, y);
+SLIM_D void set_depth_at(const DevFrame &F, uint32_t offset, float depth) {
     if (F.antialias == SLIM_AA_MSAA) {
         F.depths[offset * 4] = depth;
         F.depths[offset * 4 + 1] = 0;
@@ -1142,8 +1156,9 @@ SLIM_D void set_depth(const DevFrame &F, int x, int y, float depth) {
     }
 }
 SLIM_D void set_pixel(const DevFrame &F, int x, int y, float3 c, float depth) {
-    set_pixel_color(F, x, y, c);
-    set_depth(F, x, y, depth);
+    const uint32_t offset = canvas_offset(F, x, y);
+    set_color_at(F, offset, c);
+    set_depth_at(F, offset, depth);
 }
 
 // renderPixelBeauty (renderer/ray_tracer.h:19-108) as a sequence of path
