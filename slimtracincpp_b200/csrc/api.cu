@@ -232,7 +232,7 @@ struct Context {
         DevArray<unsigned long long> tq_masks;
         WavefrontBuffers tq{};
         cudaError_t step(const float4 *f, const float4 *t, uint32_t samples, const uint32_t *count, uint32_t offset,
-                         cudaStream_t stream) override {
+                         cudaStream_t stream, bool beside_a_frame) override {
             nrc::AdamArgs a{};
             a.lr = config.learning_rate;
             a.beta1 = config.beta1;
@@ -240,7 +240,8 @@ struct Context {
             a.eps = config.epsilon;
             a.step = state.ptr;
             return nrc::launch_train_step(f, t, samples, count, offset, params.ptr, m.ptr, v.ptr, image.ptr,
-                                          partials.ptr, loss_partials.ptr, grad.ptr, loss.ptr, a, error_flags, stream);
+                                          partials.ptr, loss_partials.ptr, grad.ptr, loss.ptr, a, error_flags, stream,
+                                          beside_a_frame);
         }
     } cache;
 };
@@ -1874,7 +1875,7 @@ int slimRadianceCacheTrain(const void *d_features, const void *d_targets, uint32
     if (!count) return SLIM_OK;
     c.cache.error_flags = c.d_error.ptr;
     cudaError_t e = c.cache.step((const float4 *)d_features, (const float4 *)d_targets, count, nullptr, 0,
-                                 (cudaStream_t)stream);
+                                 (cudaStream_t)stream, false);
     if (e != cudaSuccess) return cuda_fail(e, "cache train launch");
     return SLIM_OK;
 }

@@ -61,7 +61,7 @@ struct WavefrontBuffers {
 // the training target of the frame's Adam steps.
 struct CacheTrainer {
     virtual cudaError_t step(const float4 *features, const float4 *targets, uint32_t samples, const uint32_t *count,
-                             uint32_t offset, cudaStream_t stream) = 0;
+                             uint32_t offset, cudaStream_t stream, bool beside_a_frame = true) = 0;
     virtual ~CacheTrainer() = default;
 };
 struct CacheFrame {

@@ -1,13 +1,14 @@
 // Radiance-cache MLP kernels on the sm_100a tensor cores (tcgen05).
 //
-// One CTA of 128 threads owns a tile of 128 samples; thread t is sample row t,
+// A group of 128 threads owns a tile of 128 samples; thread t is sample row t,
 // which is also TMEM lane t of the M=128 accumulators.  Per layer one elected
 // thread issues the tcgen05.mma chain (K=16 per instruction) and commits it
 // to an mbarrier; every thread waits, reads its accumulator row with
 // tcgen05.ld, applies the activation and writes its bf16 row into the next
 // operand image in shared memory.
 //
-//   infer  forward only; 80 KB of shared memory, 128 TMEM columns, persistent
+//   infer  forward only; three groups of 128 threads per CTA, each with tiles
+//          of its own, 110 KB of shared memory, 256 TMEM columns, persistent
 //          over tiles (grid = 2 CTAs per SM).
 //   train  forward, log-radiance L2 output gradient, backward; 162 KB of shared
 //          memory (weights, the input tile, the four hidden tiles, two
@@ -41,7 +42,7 @@ using namespace umma;
 constexpr uint32_t kXBytes = kTile * kInputs * 2;    // 24576
 constexpr uint32_t kHBytes = kTile * kHidden * 2;    // 16384
 constexpr uint32_t kGBytes = kTile * kOutPad * 2;    // 4096 (output gradient tile)
-constexpr uint32_t kInferSmem = kImgBytes + kXBytes + kHBytes;                       // 79872
+constexpr uint32_t kInferSmem = kImgBytes + 3 * kXBytes;                               // 112640
 constexpr uint32_t kTrainSmem = kImgBytes + kXBytes + 4 * kHBytes + 2 * kHBytes + kGBytes;   // 165888
 
 // TMEM columns
@@ -60,7 +61,13 @@ SLIM_N uint32_t img_off(uint32_t rows, uint32_t r, uint32_t c) {
 }
 
 SLIM_N uint32_t bf16_bits(float x) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x)); }
-SLIM_N uint32_t pack2(float a, float b) { return bf16_bits(a) | (bf16_bits(b) << 16); }
+// Both roundings in one instruction: a conversion of its own each kept the
+// special-function pipe busy for 107 of a query's 149 us.
+SLIM_N uint32_t pack2(float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
 SLIM_N float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 SLIM_N float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
@@ -99,6 +106,12 @@ SLIM_N void tmem_ld16w(uint32_t taddr, float v[16]) {
                  : "r"(taddr) : "memory");
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 32 floats of a 16-byte aligned gradient row.
+SLIM_N void store32(float *out, const float v[32]) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *(float4 *)(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
 }
 
 // Real spherical harmonics, bands 0..3, of a unit vector.
@@ -197,74 +210,100 @@ SLIM_N void sync_for_mma() {
 }
 
 // ---- inference --------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_nrc_infer(const float4 *__restrict__ features, const uint32_t *count,
-                                                   uint32_t n_host, float4 *__restrict__ radiance,
-                                                   const uint8_t *__restrict__ weight_image, uint32_t *error_flags) {
+// What bounds a tile is its chain -- features, encoding, five times MMA, wait,
+// epilogue -- about 7 us for one group of four warps, with the tensor cores
+// and the issue slots almost idle.  So six tiles are in flight per SM: two
+// CTAs of three groups, each group a tile and a chain of its own, over one
+// copy of the weights per CTA.  A tile's hidden rows take the place of its
+// input rows, which are dead after the first layer, and all its layers share
+// 64 TMEM columns: 24 KB of shared memory and an eighth of the columns a tile.
+// 1,036,801 samples: 196 us with two tiles per SM, 149 us with six, 102 us with
+// packed conversions (pack2) besides.
+constexpr uint32_t kGroups = 3;
+SLIM_N void group_sync(uint32_t group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory"); }
+SLIM_N void group_sync_for_mma(uint32_t group) {
+    fence_smem_to_async();
+    fence_before_sync();
+    group_sync(group);
+    fence_after_sync();
+}
+
+__global__ void __launch_bounds__(128 * kGroups, 2) k_nrc_infer(const float4 *__restrict__ features,
+                                                                const uint32_t *count, uint32_t n_host,
+                                                                float4 *__restrict__ radiance,
+                                                                const uint8_t *__restrict__ weight_image,
+                                                                uint32_t *error_flags) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *W = smem, *X = smem + kImgBytes, *H = X + kXBytes;
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bars[kGroups];
     __shared__ uint32_t tmem_base_s;
-    __shared__ int abort_s;
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+    __shared__ int abort_s[kGroups];
+    const uint32_t group = threadIdx.x >> 7, t = threadIdx.x & 127u, warp = t >> 5;
+    uint8_t *W = smem, *X = smem + kImgBytes + group * kXBytes;      // rows of X, then of H1..H4
     const uint32_t n = count ? *count : n_host;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     if (blockIdx.x >= tiles) return;                       // uniform over the CTA, before any allocation
-    for (uint32_t i = t; i < kImgBytes / 16; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i < kImgBytes / 16; i += blockDim.x)
         ((uint4 *)W)[i] = ((const uint4 *)weight_image)[i];
-    if (t == 0) { mbar_init(&bar, 1); abort_s = 0; }
-    if (warp == 0) tmem_alloc(&tmem_base_s, 128);
+    if (t == 0) { mbar_init(&bars[group], 1); abort_s[group] = 0; }
+    if (threadIdx.x < 32u) tmem_alloc(&tmem_base_s, 256);
     sync_for_mma();
-    const uint32_t tb = tmem_base_s;
+    const uint32_t tb = tmem_base_s + group * (uint32_t)kHidden;
     const uint32_t lane = tmem_at(tb, warp * 32u, 0);
-    const uint32_t sW = smem_addr(W), sX = smem_addr(X), sH = smem_addr(H);
+    const uint32_t sW = smem_addr(W), sX = smem_addr(X);
+    uint64_t *bar = &bars[group];
     uint32_t phase = 0;
     bool aborted = false;
-    for (uint32_t tile = blockIdx.x; tile < tiles && !aborted; tile += gridDim.x) {
+    // tiles go round the CTAs first, so few tiles spread over the SMs
+    for (uint32_t tile = group * gridDim.x + blockIdx.x; tile < tiles && !aborted; tile += kGroups * gridDim.x) {
         const uint32_t i = tile * kTile + t;
         const bool valid = i < n;
         encode_row(features + 4 * (size_t)i, valid, X, t);
-        sync_for_mma();
+        group_sync_for_mma(group);
         for (int l = 0; l < 5; l++) {
             if (t == 0) {
                 if (l == 0) {
 #pragma unroll
                     for (uint32_t k = 0; k < kInputs / 16; k++)
-                        mma(tb + kColFwd, kmajor(sX, kTile, k), kmajor(sW, kHidden, k), kIdHidden0, k > 0);
+                        mma(tb, kmajor(sX, kTile, k), kmajor(sW, kHidden, k), kIdHidden0, k > 0);
                 } else if (l < 4) {
                     const uint32_t w = sW + kImgOff1 + (l - 1) * kImgW;
 #pragma unroll
                     for (uint32_t k = 0; k < kHidden / 16; k++)
-                        mma(tb + kColFwd, kmajor(sH, kTile, k), kmajor(w, kHidden, k), kIdHidden0, k > 0);
+                        mma(tb, kmajor(sX, kTile, k), kmajor(w, kHidden, k), kIdHidden0, k > 0);
                 } else {
 #pragma unroll
                     for (uint32_t k = 0; k < kHidden / 16; k++)
-                        mma(tb + kColOut, kmajor(sH, kTile, k), kmajor(sW + kImgOff4, kOutPad, k), kIdOut, k > 0);
+                        mma(tb, kmajor(sX, kTile, k), kmajor(sW + kImgOff4, kOutPad, k), kIdOut, k > 0);
                 }
-                commit(&bar);
+                commit(bar);
             }
-            if (!mbar_wait(&bar, phase)) abort_s = 1;
+            if (!mbar_wait(bar, phase)) abort_s[group] = 1;
             phase ^= 1u;
             fence_after_sync();
             if (l < 4) {
-                epilogue_relu(lane + kColFwd, H, t);
+                epilogue_relu(lane, X, t);
             } else {
                 float z[16];
-                tmem_ld16w(lane + kColOut, z);
+                tmem_ld16w(lane, z);
                 if (valid)
                     radiance[i] = make_float4(fmaxf(expf(fminf(z[0], kZMax)) - kLogOffset, 0.0f),
                                               fmaxf(expf(fminf(z[1], kZMax)) - kLogOffset, 0.0f),
                                               fmaxf(expf(fminf(z[2], kZMax)) - kLogOffset, 0.0f), 0.0f);
             }
-            sync_for_mma();
-            if (abort_s) { aborted = true; break; }
+            group_sync_for_mma(group);
+            if (abort_s[group]) { aborted = true; break; }
         }
     }
-    if (aborted) {
-        if (t == 0) { atomicOr(error_flags, kErrTimeout); mbar_wait(&bar, phase); }
-        fence_before_sync();
-        __syncthreads();
+    if (aborted && t == 0) {
+        atomicOr(error_flags, kErrTimeout);
+        mbar_wait(bar, phase);
     }
-    if (warp == 0) tmem_free(tb, 128);
+    fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        fence_after_sync();
+        tmem_free(tmem_base_s, 256);
+    }
 }
 
 // ---- training -----------------------------------------------------------------
@@ -434,15 +473,13 @@ __global__ void __launch_bounds__(128, 1) k_nrc_train(const float4 *__restrict__
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             tmem_ld32(lane + kColDW0 + 32u * c, v);
-            if (has_row)
-                for (int j = 0; j < 32; j++) out[row * kInputs + 32 * c + j] = v[j];
+            if (has_row) store32(out + row * kInputs + 32 * c, v);
         }
         for (int l = 0; l < 3; l++) {
 #pragma unroll
             for (int c = 0; c < 2; c++) {
                 tmem_ld32(lane + kColDW1 + 64u * l + 32u * c, v);
-                if (has_row)
-                    for (int j = 0; j < 32; j++) out[kParamsW0 + l * kParamsW + row * kHidden + 32 * c + j] = v[j];
+                if (has_row) store32(out + kParamsW0 + l * kParamsW + row * kHidden + 32 * c, v);
             }
         }
         float v16[16];
@@ -471,25 +508,40 @@ SLIM_N uint32_t param_offset(uint32_t p) {
     return kImgOff4 + img_off(kOutPad, p / kHidden, p % kHidden);
 }
 
-__global__ void k_nrc_adam(float *__restrict__ params, float *__restrict__ m, float *__restrict__ v,
-                           const float *__restrict__ partials, const float *__restrict__ loss_partials,
-                           float *__restrict__ grad, float *__restrict__ loss, uint8_t *__restrict__ image, AdamArgs a,
-                           uint32_t n_max, const uint32_t *count, uint32_t offset) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+// Sums the partial rows and updates the parameters.  What bounds it is the
+// latency of the rows' loads (9.5 MB for a 16,384-sample step of 128 CTAs), so
+// four threads share a parameter, each a quarter of the rows in order, and the
+// quarters are added in a fixed order: 14.9 -> 8.7 us cold.
+constexpr uint32_t kAdamParams = 64, kAdamParts = 4;
+__global__ void __launch_bounds__(kAdamParams * kAdamParts) k_nrc_adam(
+    float *__restrict__ params, float *__restrict__ m, float *__restrict__ v, const float *__restrict__ partials,
+    const float *__restrict__ loss_partials, float *__restrict__ grad, float *__restrict__ loss,
+    uint8_t *__restrict__ image, AdamArgs a, uint32_t n_max, const uint32_t *count, uint32_t offset) {
+    __shared__ float quarter[kAdamParts][kAdamParams];
+    const uint32_t k = threadIdx.x % kAdamParams, q = threadIdx.x / kAdamParams;
+    const uint32_t p = blockIdx.x * kAdamParams + k;
     const uint32_t n = step_samples(n_max, count, offset);
     if (!n) return;                                  // empty step: no update
+    const uint32_t rows = (a.parts + kAdamParts - 1) / kAdamParts, first = q * rows;
+    const uint32_t end = min(first + rows, a.parts);
+    float g = 0.0f;
+    if (p < (uint32_t)kParams) {
+#pragma unroll 8
+        for (uint32_t b = first; b < end; b++) g += partials[(size_t)b * kParams + p];
+    }
+    quarter[q][k] = g;
+    __syncthreads();
     const float scale = 1.0f / (3.0f * (float)n);
-    const float t = (float)*a.step;
-    const float bias1 = 1.0f / (1.0f - powf(a.beta1, t)), bias2 = 1.0f / (1.0f - powf(a.beta2, t));
-    if (p == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == kAdamParams) {
         float s = 0.0f;
+#pragma unroll 8
         for (uint32_t b = 0; b < a.parts; b++) s += loss_partials[b];
         *loss = s * scale;
     }
-    if (p >= (uint32_t)kParams) return;
-    float g = 0.0f;
-    for (uint32_t b = 0; b < a.parts; b++) g += partials[(size_t)b * kParams + p];
-    g *= scale;
+    if (q || p >= (uint32_t)kParams) return;
+    g = ((quarter[0][k] + quarter[1][k]) + (quarter[2][k] + quarter[3][k])) * scale;
+    const float t = (float)*a.step;
+    const float bias1 = 1.0f / (1.0f - powf(a.beta1, t)), bias2 = 1.0f / (1.0f - powf(a.beta2, t));
     grad[p] = g;
     float mm = a.beta1 * m[p] + (1.0f - a.beta1) * g;
     float vv = a.beta2 * v[p] + (1.0f - a.beta2) * g * g;
@@ -523,14 +575,17 @@ int sm_count() {
 // the L1 cache that the traversal kernels running beside an overlapped
 // training step read their nodes through: config 4 (65,536 samples per
 // frame) 1.694 ms per cache frame with 128 CTAs per step, 1.648 with 64,
-// 1.636 with 32.
+// 1.636 with 32.  A step of its own (slimRadianceCacheTrain) has the GPU to
+// itself and takes a CTA per tile: 16,384 samples with their gradients read
+// back 115 -> 87 us (75 us with gradient rows stored 16 bytes at a time and
+// Adam's sums split).
 #ifndef SLIM_NRC_TRAIN_MAX_CTAS
 #define SLIM_NRC_TRAIN_MAX_CTAS 32
 #endif
-int train_grid(uint32_t samples) {
+int train_grid(uint32_t samples, bool beside_a_frame) {
     uint32_t tiles = (samples + kTile - 1) / kTile;
     uint32_t g = (uint32_t)sm_count();
-    if (SLIM_NRC_TRAIN_MAX_CTAS > 0 && g > (uint32_t)SLIM_NRC_TRAIN_MAX_CTAS) g = SLIM_NRC_TRAIN_MAX_CTAS;
+    if (beside_a_frame && SLIM_NRC_TRAIN_MAX_CTAS > 0 && g > (uint32_t)SLIM_NRC_TRAIN_MAX_CTAS) g = SLIM_NRC_TRAIN_MAX_CTAS;
     return (int)(tiles < g ? (tiles ? tiles : 1) : g);
 }
 
@@ -547,7 +602,7 @@ cudaError_t launch_infer(const float4 *features, const uint32_t *count, uint32_t
     if (!tiles) return cudaSuccess;
     uint32_t g = 2u * (uint32_t)sm_count();
     if (tiles < g) g = tiles;
-    k_nrc_infer<<<g, 128, kInferSmem, stream>>>(features, count, n, radiance, weight_image, error_flags);
+    k_nrc_infer<<<g, 128 * kGroups, kInferSmem, stream>>>(features, count, n, radiance, weight_image, error_flags);
     count_launch();
     return cudaGetLastError();
 }
@@ -555,15 +610,15 @@ cudaError_t launch_infer(const float4 *features, const uint32_t *count, uint32_t
 cudaError_t launch_train_step(const float4 *features, const float4 *targets, uint32_t samples, const uint32_t *count,
                               uint32_t offset, float *params, float *adam_m, float *adam_v, uint8_t *weight_image,
                               float *partials, float *loss_partials, float *grad, float *loss, const AdamArgs &adam,
-                              uint32_t *error_flags, cudaStream_t stream) {
+                              uint32_t *error_flags, cudaStream_t stream, bool beside_a_frame) {
     if (!samples) return cudaSuccess;
-    int g = train_grid(samples);
+    int g = train_grid(samples, beside_a_frame);
     k_nrc_train<<<g, 128, kTrainSmem, stream>>>(features, targets, samples, count, offset, weight_image, partials,
                                                  loss_partials, adam.step, error_flags);
     count_launch();
     AdamArgs a = adam;
     a.parts = (uint32_t)g;
-    k_nrc_adam<<<(kParams + 255) / 256, 256, 0, stream>>>(params, adam_m, adam_v, partials, loss_partials, grad, loss,
+    k_nrc_adam<<<(kParams + kAdamParams - 1) / kAdamParams, kAdamParams * kAdamParts, 0, stream>>>(params, adam_m, adam_v, partials, loss_partials, grad, loss,
                                                           weight_image, a, samples, count, offset);
     count_launch();
     return cudaGetLastError();

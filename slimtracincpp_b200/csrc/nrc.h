@@ -46,8 +46,9 @@ struct AdamArgs {
 // Sets the kernels' shared-memory limits (before any launch or graph capture).
 cudaError_t prepare();
 
-// Largest grid the training kernel uses (rows of the partial-gradient buffer).
-int train_grid(uint32_t samples);
+// Grid of the training kernel (rows of the partial-gradient buffer it fills),
+// at most the SM count; fewer CTAs for a step that runs beside a frame.
+int train_grid(uint32_t samples, bool beside_a_frame);
 
 // radiance[i] = cache(features[i]) for i < n; n = *count when count is given.
 cudaError_t launch_infer(const float4 *features, const uint32_t *count, uint32_t n, uint32_t capacity,
@@ -61,7 +62,7 @@ cudaError_t launch_infer(const float4 *features, const uint32_t *count, uint32_t
 cudaError_t launch_train_step(const float4 *features, const float4 *targets, uint32_t samples, const uint32_t *count,
                               uint32_t offset, float *params, float *adam_m, float *adam_v, uint8_t *weight_image,
                               float *partials, float *loss_partials, float *grad, float *loss, const AdamArgs &adam,
-                              uint32_t *error_flags, cudaStream_t stream);
+                              uint32_t *error_flags, cudaStream_t stream, bool beside_a_frame);
 
 // bf16 image of `params` (after the host sets the weights).
 cudaError_t launch_pack_weights(const float *params, uint8_t *weight_image, cudaStream_t stream);
