@@ -789,7 +789,7 @@ int cache_frame(Context &c, uint32_t samples, CacheFrame &cf) {
         if ((rc = k.tq_hits.reserve(3 * (size_t)cap, "alloc training queues"))) return rc;
         if ((rc = k.tq_shadow.reserve(2 * shadow, "alloc training queues"))) return rc;
         if ((rc = k.tq_pairs.reserve(3 * pairs, "alloc training queues"))) return rc;
-        if ((rc = k.tq_counts.reserve(8, "alloc training queues"))) return rc;
+        if ((rc = k.tq_counts.reserve(kCounterWords, "alloc training queues"))) return rc;
         if ((rc = k.tq_masks.reserve(cap, "alloc training queues"))) return rc;
         if ((rc = k.image_infer.reserve(nrc::kImgBytes, "alloc weight snapshot"))) return rc;
         WavefrontBuffers &T = k.tq;
@@ -945,7 +945,7 @@ int ensure_wavefront(Context &c, uint32_t samples, int set) {
     if ((rc = W.rays1.reserve(2 * (size_t)n, "alloc ray queue"))) return rc;
     if ((rc = W.hits.reserve(3 * (size_t)n, "alloc hit records"))) return rc;
     if ((rc = W.shadow_rays.reserve(2 * shadow, "alloc shadow queue"))) return rc;
-    if ((rc = W.counts.reserve(8, "alloc queue counters"))) return rc;
+    if ((rc = W.counts.reserve(kCounterWords, "alloc queue counters"))) return rc;
     if ((rc = W.mask.reserve(n, "alloc shadow masks"))) return rc;
     if ((rc = W.pairs.reserve(3 * (pairs ? pairs : 1), "alloc shadow candidate pairs"))) return rc;
     WavefrontBuffers &B = W.B;
@@ -1564,7 +1564,8 @@ namespace {
 
 constexpr size_t kNoAllocScratchBytes = 64ull << 20;   // held by every GPU that loads the library
 constexpr int kNoAllocMaxDevices = 64;
-__device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+// the queues, then the rounds' counters
+__device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kCounterWords * sizeof(uint32_t)];
 unsigned char *g_noalloc_base[kNoAllocMaxDevices] = {};
 
 // Device address of this device's copy of the array, looked up once per
@@ -1599,7 +1600,8 @@ int noalloc_layout(unsigned char *base, uint32_t samples, uint32_t lights, Wavef
     B.rays[1] = (float4 *)take(32 * n);
     B.hits = (float4 *)take(48 * n);
     B.shadow_mask = (unsigned long long *)take(8 * n);
-    B.queue_count = (uint32_t *)take(8 * sizeof(uint32_t));
+    take(8 * sizeof(uint32_t));
+    B.queue_count = (uint32_t *)(base + kNoAllocScratchBytes);
     if (off > kNoAllocScratchBytes) return set_error(SLIM_ERR_LIMIT, "frame larger than the no-alloc scratch (64 MiB)");
     size_t left = kNoAllocScratchBytes - off;
     size_t per_light = n * (32 + 48);           // one shadow ray + at least one candidate pair per sample and light
@@ -2056,7 +2058,7 @@ int ensure_batch_queues(BatchState &b) {
         if ((rc = u.hits.reserve(3 * Q, "alloc batch hits"))) return rc;
         if ((rc = u.shadow_rays.reserve(2 * shadow, "alloc batch shadow rays"))) return rc;
         if ((rc = u.pairs.reserve(3 * pairs, "alloc batch shadow pairs"))) return rc;
-        if ((rc = u.counts.reserve(8, "alloc batch counters"))) return rc;
+        if ((rc = u.counts.reserve(kCounterWords, "alloc batch counters"))) return rc;
         if ((rc = u.masks.reserve(Q, "alloc batch masks"))) return rc;
         WavefrontBuffers &B = u.B;
         B.path_color = u.color.ptr;

@@ -110,7 +110,8 @@ struct QueueArgs {
     const float4 *rays_in;        // null: primary rays generated from the slot (= sample index)
     float4 *rays_out;
     const uint32_t *count_in;     // null: count = samples
-    uint32_t *count_out;
+    uint32_t *count_out;          // between rounds: the rays queued for the next
+    uint32_t *round_counts;       // the next round's counters
     float4 *hits;                 // hit records, three planes of hit_stride entries
     uint32_t hit_stride;
     float4 *shadow_rays;
@@ -1623,7 +1624,7 @@ cudaError_t tail_round(const RoundLaunch &L, QueueArgs &A, uint32_t in, uint32_t
     const WavefrontBuffers &B = *L.B;
     A.depth = depth;
     A.rays_in = B.rays[in];
-    A.count_in = B.queue_count + in;
+    A.count_in = A.count_out;
     if (L.pixel_wait) {
         cudaError_t r = cudaStreamWaitEvent(L.stream, L.pixel_wait, 0);
         if (r != cudaSuccess) return r;
@@ -1649,22 +1650,21 @@ cudaError_t trace_round(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
     StageTimer *timer = L.timer;
     uint32_t out = in ^ 1u;
     A.depth = depth;
+    uint32_t *const counts = A.round_counts;
+    A.round_counts += kRoundWords;
     A.rays_in = primary ? nullptr : B.rays[in];
-    A.count_in = primary ? nullptr : B.queue_count + in;
+    A.count_in = primary ? nullptr : A.count_out;
     A.rays_out = B.rays[out];
-    A.count_out = B.queue_count + out;
-    // the output queue of this round is the input of the next: clear it
-    cudaError_t r = cudaMemsetAsync(B.queue_count + out, 0, sizeof(uint32_t), stream);
-    if (r != cudaSuccess) return r;
+    A.count_out = counts;
+    cudaError_t r;
     A.counters = L.stage(STAGE_EXTEND);
     if (timer) timer->begin(STAGE_EXTEND, stream);
     if (hits_given) {
         // the queued rays' hit records are in place already (training paths
         // that start at their cache vertex)
     } else if (L.split_extend && B.pair_capacity >= 4) {
-        // [3] candidates, [4] candidate cursor, [5] rays traced whole, [6] records of parts of walks
-        r = cudaMemsetAsync(B.queue_count + 3, 0, 4 * sizeof(uint32_t), stream);
-        if (r != cudaSuccess) return r;
+        A.pair_count = counts + 1;
+        A.pair_cursor = counts + 2;
         k_extend_scene<COUNT, BATCH><<<L.grid((const void *)k_extend_scene<COUNT, BATCH>, L.bound), L.block, 0, stream>>>(S, F, A);
         count_launch();
         k_extend_mesh<COUNT><<<L.mesh_grid((const void *)k_extend_mesh<COUNT>, B.pair_capacity), kMeshBlock, 0,
@@ -1694,9 +1694,8 @@ cudaError_t trace_round(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
     for (uint32_t l0 = 0; l0 < L.lights; l0 += per_batch) {
         A.light_begin = l0;
         A.light_end = l0 + per_batch < L.lights ? l0 + per_batch : L.lights;
-        r = cudaMemsetAsync(B.queue_count + 2, 0, sizeof(uint32_t), stream);
-        if (r != cudaSuccess) return r;
-        A.shadow_count = B.queue_count + 2;
+        if (l0 && (r = cudaMemsetAsync(counts + 5, 0, 3 * sizeof(uint32_t), stream)) != cudaSuccess) return r;
+        A.shadow_count = counts + 5;
         A.counters = L.stage(STAGE_SHADOW_GEN);
         if (timer) timer->begin(STAGE_SHADOW_GEN, stream);
         k_shadow_gen<COUNT, BATCH><<<L.grid((const void *)k_shadow_gen<COUNT, BATCH>, L.bound), L.block, 0, stream>>>(S, F, A);
@@ -1711,10 +1710,10 @@ cudaError_t trace_round(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
                 return r;
         }
         // Scene arrays without meshes (split_extend is false exactly then)
-        // append no (shadow ray, instance) pairs: no pair counters, no mesh pass
-        // (config 3: 0.021 ms of a 0.56 ms whole-frame pass).
-        if (L.split_extend && (r = cudaMemsetAsync(B.queue_count + 3, 0, 2 * sizeof(uint32_t), stream)) != cudaSuccess)
-            return r;
+        // append no (shadow ray, instance) pairs: no mesh pass (config 3: 0.021
+        // ms of a 0.56 ms whole-frame pass).
+        A.pair_count = counts + 6;
+        A.pair_cursor = counts + 7;
         A.counters = L.stage(STAGE_SHADOW);
         if (timer) timer->begin(STAGE_SHADOW, stream);
         k_shadow_scene<COUNT, BATCH><<<L.grid((const void *)k_shadow_scene<COUNT, BATCH>, L.bound * (A.light_end - A.light_begin)),
@@ -1852,7 +1851,7 @@ cudaError_t cache_phase(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         if ((e = cudaMemcpyAsync((void *)cache->weights, cache->train_weights, nrc::kImgBytes, cudaMemcpyDeviceToDevice,
                                  stream)) != cudaSuccess)
             return e;
-        if ((e = cudaMemsetAsync(TB.queue_count, 0, 8 * sizeof(uint32_t), stream)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(TB.queue_count, 0, counter_bytes(max_depth + 2), stream)) != cudaSuccess) return e;
         if (timer) timer->begin(STAGE_CACHE, stream);
         uint32_t g = (cache->train_capacity + 255) / 256;
         if (g > (uint32_t)(L.sms * 8)) g = (uint32_t)(L.sms * 8);
@@ -1869,8 +1868,8 @@ cudaError_t cache_phase(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         TA.shadow_rays = TB.shadow_rays;
         TA.masks = TB.shadow_mask;
         TA.pairs = TB.pairs;
-        TA.pair_count = TB.queue_count + 3;
-        TA.pair_cursor = TB.queue_count + 4;
+        TA.count_out = TB.queue_count;
+        TA.round_counts = TB.queue_count + kRoundWords;
         TA.pair_capacity = TB.pair_capacity;
         TA.path_color = cache->t_color;
         TA.path_throughput = cache->t_through;
@@ -1895,6 +1894,7 @@ cudaError_t cache_phase(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         if (timer) timer->end(STAGE_CACHE, stream);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         QueueArgs main = A;
+        A.count_out = B.queue_count + in;
         A.path_color = cache->t_color;
         A.path_throughput = cache->t_through;
         A.sink = cache->t_targets;
@@ -1902,6 +1902,7 @@ cudaError_t cache_phase(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         if ((e = trace_training<COUNT, BATCH>(L, A, CA, in, cache, max_depth,
                                               mode == SLIM_CACHE_ON ? cache->weights : nullptr)) != cudaSuccess)
             return e;
+        main.round_counts = A.round_counts;
         A = main;
     }
     if (train && !(cache->train_stream && cache->train_queues && !BATCH)) {
@@ -1942,7 +1943,7 @@ cudaError_t run_frame(const DevScene &S, const DevFrame &F, const WavefrontBuffe
     // the cache's overlapped training runs beside this frame: leave it room
     // (config 4: 3.50 -> 3.37 ms per frame)
     L.share_sms = cache && cache->train_stream && cache->mode == SLIM_CACHE_ON && !cache->train_suffix;
-    cudaError_t e = cudaMemsetAsync(B.queue_count, 0, 8 * sizeof(uint32_t), stream);
+    cudaError_t e = cudaMemsetAsync(B.queue_count, 0, counter_bytes(2 * F.settings.max_depth + 4), stream);
     if (e != cudaSuccess) return e;
     QueueArgs A{};
     A.hits = B.hits;
@@ -1950,8 +1951,7 @@ cudaError_t run_frame(const DevScene &S, const DevFrame &F, const WavefrontBuffe
     A.shadow_rays = B.shadow_rays;
     A.masks = B.shadow_mask;
     A.pairs = B.pairs;
-    A.pair_count = B.queue_count + 3;
-    A.pair_cursor = B.queue_count + 4;
+    A.round_counts = B.queue_count + kRoundWords;
     A.pair_capacity = B.pair_capacity;
     A.path_color = B.path_color;
     A.path_throughput = B.path_throughput;
@@ -2047,7 +2047,7 @@ cudaError_t run_batch(const BatchFrame &BF, const WavefrontBuffers &B0, int bloc
         const cudaStream_t stream = lane ? BF.lane_stream : stream0;
         RoundLaunch L{&BF.shared, &BF.frame, &B, block <= 0 ? 256 : block, sms, stream, timer, BF.frame.counters,
                       B.capacity, wave.max_lights, BF.shared.mesh_count > 0};
-        if ((e = cudaMemsetAsync(B.queue_count, 0, 8 * sizeof(uint32_t), stream)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(B.queue_count, 0, counter_bytes(2 * wave.max_depth + 4), stream)) != cudaSuccess) return e;
         const bool use_cache = cache && wave.cache_paths;
         if (use_cache && (e = cudaMemsetAsync(cache->counts, 0, sizeof(uint32_t), stream)) != cudaSuccess)
             return e;
@@ -2057,8 +2057,8 @@ cudaError_t run_batch(const BatchFrame &BF, const WavefrontBuffers &B0, int bloc
         A.shadow_rays = B.shadow_rays;
         A.masks = B.shadow_mask;
         A.pairs = B.pairs;
-        A.pair_count = B.queue_count + 3;
-        A.pair_cursor = B.queue_count + 4;
+        A.count_out = B.queue_count;
+        A.round_counts = B.queue_count + kRoundWords;
         A.pair_capacity = B.pair_capacity;
         A.path_color = B.path_color;
         A.path_throughput = B.path_throughput;
