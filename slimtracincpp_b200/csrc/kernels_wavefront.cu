@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
     Feed feed(min(*A.pair_count, A.pair_capacity));
     uint32_t stack[kStackCapacity];
     Work w = {};
-    bool busy = false;
+    bool busy = false, hit = false;
     uint32_t idx = 0, tag = 0, top = 0, bottom = 0, tri_offset = 0;
     uint32_t next = kNone;          // node or leaf the walk goes to
     uint32_t waiting = kNone;       // a leaf to be tested
@@ -643,6 +643,17 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
         advance();
     };
     for (;;) {
+        // an occluded ray ends its other parts and pairs in this warp too
+        // (8 bounces 2.150 -> 2.139 ms)
+        for (uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit); hits; hits &= hits - 1u) {
+            const uint32_t occluded = __shfl_sync(0xFFFFFFFFu, tag, __ffs((int)hits) - 1);     // every lane takes part
+            if (busy && tag == occluded) {
+                busy = false;
+                next = waiting = kNone;
+                top = bottom = 0;
+            }
+        }
+        hit = false;
         const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
         if (idle) {
             const uint32_t donors = feed.donors(busy && top > bottom);
@@ -690,6 +701,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
             waiting = kNone;
             if (wide_leaf_box(r, wr, a, b, ln, lf) && ln < aux && any_triangle<COUNT>(S, leaf, tri_offset, b, minr(lf, aux), r, w)) {
                 atomicOr(A.masks + (tag >> 6), 1ull << (tag & 63u));
+                hit = true;
                 next = kNone;
                 top = bottom = 0;
             }
