@@ -14,6 +14,8 @@
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "slimtracer_b200.h"
 #include "device_scene.h"
@@ -82,9 +84,18 @@ class HostCopyPool {
         for (std::thread &t : threads_) t.join();
     }
     // dst[0, bytes) = src[0, bytes), split over the pool; returns when done.
-    void copy(void *dst, const void *src, size_t bytes) {
+    void copy(void *dst, const void *src, size_t bytes) { run((char *)dst, (const char *)src, bytes); }
+    // Gives [dst, dst + bytes) its pages, contents unchanged, split over the
+    // pool: a canvas fresh from the allocator has none, and the faults, taken
+    // while the frame renders, are not left for the copy.  A kernel without the
+    // call, or memory it refuses, leaves them to the copy as before.
+    void populate(void *dst, size_t bytes) { run((char *)dst, nullptr, bytes); }
+
+  private:
+    static constexpr size_t kChunk = 1 << 20;
+    void run(char *dst, const char *src, size_t bytes) {
         if (bytes < kChunk) {
-            memcpy(dst, src, bytes);
+            part(dst, src, bytes);
             return;
         }
         std::unique_lock<std::mutex> lock(m_);
@@ -93,8 +104,8 @@ class HostCopyPool {
             n = n < 2 ? 2 : (n > 16 ? 16 : n);
             for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
         }
-        dst_ = (char *)dst;
-        src_ = (const char *)src;
+        dst_ = dst;
+        src_ = src;
         bytes_ = bytes;
         next_ = 0;
         busy_ = (uint32_t)threads_.size();
@@ -102,9 +113,16 @@ class HostCopyPool {
         start_.notify_all();
         done_.wait(lock, [this] { return busy_ == 0; });
     }
-
-  private:
-    static constexpr size_t kChunk = 1 << 20;
+    static void part(char *dst, const char *src, size_t bytes) {
+        if (src) {
+            memcpy(dst, src, bytes);
+            return;
+        }
+#ifdef MADV_POPULATE_WRITE
+        const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = (uintptr_t)dst & ~(page - 1);
+        madvise((void *)first, ((uintptr_t)dst + bytes + page - 1 & ~(page - 1)) - first, MADV_POPULATE_WRITE);
+#endif
+    }
     void work() {
         uint64_t seen = 0;
         for (;;) {
@@ -118,7 +136,7 @@ class HostCopyPool {
                 next_ = off + kChunk;
                 const size_t n = std::min(kChunk, bytes_ - off);
                 lock.unlock();
-                memcpy(dst_ + off, src_ + off, n);
+                part(dst_ + off, src_ ? src_ + off : nullptr, n);
                 lock.lock();
             }
             if (--busy_ == 0) done_.notify_one();
@@ -1348,6 +1366,10 @@ int slimRenderOnGPU(const SlimCanvasData *canvas, const SlimCameraRayProjection 
     if ((rc = render_frame(c, canvas, projection, settings, c.d_pixels.ptr, c.d_depths.ptr, c.stream, host_pixels,
                            host_depths, pixel_count, depth_count)))
         return rc;
+    if (staged) {
+        c.copy_pool.populate(canvas->pixels, pixel_bytes);
+        c.copy_pool.populate(canvas->depths, depth_bytes);
+    }
     if ((rc = read_errors(c, c.stream))) return rc;
     if (staged) {
         c.copy_pool.copy(canvas->pixels, host_pixels, pixel_bytes);

@@ -29,10 +29,13 @@ class Viewport:
         return self.antialias == L.AA_SSAA
 
 
-def make_canvas(width, height, antialias):
+def make_canvas(width, height, antialias, cleared=True):
+    """`cleared`: black pixels and infinite depths; a frame writes every entry
+    of both, so its own canvas needs neither."""
     s = 2 if antialias == L.AA_SSAA else 1
-    pixels = np.zeros((height * s * width * s, 4), np.float32)
-    depths = np.full(height * width * (1 if antialias == L.AA_NONE else 4), np.inf, np.float32)
+    entries = height * width * (1 if antialias == L.AA_NONE else 4)
+    pixels = (np.zeros if cleared else np.empty)((height * s * width * s, 4), np.float32)
+    depths = np.full(entries, np.inf, np.float32) if cleared else np.empty(entries, np.float32)
     cv = np.zeros((), L.CANVAS_DATA)
     cv["width_times_height"] = width * height
     cv["f_width"], cv["f_height"] = width, height
@@ -69,7 +72,7 @@ class RayTracingRenderer:
         if update_scene:
             self.scene.build_bvh()
             self.upload()
-        cv, pixels, depths = make_canvas(viewport.width, viewport.height, viewport.antialias)
+        cv, pixels, depths = make_canvas(viewport.width, viewport.height, viewport.antialias, cleared=False)
         proj = viewport.camera.projection(viewport.width, viewport.height, viewport.ssaa)
         check(lib().slimRenderOnGPU(ptr(cv), ptr(proj), ptr(self.settings)))
         return pixels, depths
