@@ -30,15 +30,16 @@ uint32_t to_bits(float f) {
 // decodes to x or more.  (Offset 0 with bits below reads as a denormal,
 // which the walk's margin covers.)
 uint32_t plane_bits(double x, bool up, uint32_t below) {
-    uint32_t h = to_bits((float)x) >> 16;
+    const float f = (float)x;
+    uint32_t bits = to_bits(f);                      // floats of one sign order as their bits
     if (up) {
-        while (h && (double)from_bits((h - 1) << 16 | below) >= x) h--;
-        while ((double)from_bits(h << 16 | below) < x) h++;
-    } else {
-        while ((double)from_bits((h + 1) << 16 | below) <= x) h++;
-        while (h && (double)from_bits(h << 16 | below) > x) h--;
+        if ((double)f < x) bits++;
+        const uint32_t h = bits >> 16;
+        return (h << 16 | below) < bits ? h + 1 : h;
     }
-    return h;
+    if ((double)f > x) bits--;
+    const uint32_t h = bits >> 16;
+    return h && (h << 16 | below) > bits ? h - 1 : h;
 }
 
 double surface(const SlimBVHNode &n) {
@@ -76,19 +77,28 @@ uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const flo
     const size_t root = out.size(), first_leaf = leaves.size();
     std::vector<uint32_t> source{0};       // binary node of every wide node from `root` on
     std::vector<uint32_t> waiting{0};      // nodes a walk may have waiting when it enters it
+    source.reserve(node_count / 2);
+    waiting.reserve(node_count / 2);
+    out.reserve(root + node_count / 3);
+    leaves.reserve(first_leaf + node_count / 2 + 1);
     for (size_t w = 0; w < source.size(); w++) {
         // open the largest inner child until four are reached
-        uint32_t child[4] = {nodes[source[w]].first_index, nodes[source[w]].first_index + 1};
-        uint32_t count = 2;
+        uint32_t child[4], count = 0;
+        double area[4];                              // of an inner child's box; a leaf is not opened
+        auto put = [&](uint32_t k, uint32_t node) {
+            child[k] = node;
+            area[k] = nodes[node].leaf_count ? -1.0 : surface(nodes[node]);
+        };
+        put(count++, nodes[source[w]].first_index);
+        put(count++, nodes[source[w]].first_index + 1);
         while (count < 4) {
-            int open = -1;
-            for (uint32_t k = 0; k < count; k++)
-                if (!nodes[child[k]].leaf_count && (open < 0 || surface(nodes[child[k]]) > surface(nodes[child[open]])))
-                    open = (int)k;
-            if (open < 0) break;
+            uint32_t open = 0;
+            for (uint32_t k = 1; k < count; k++)
+                if (area[k] > area[open]) open = k;
+            if (area[open] < 0.0) break;
             const uint32_t first = nodes[child[open]].first_index;
-            child[open] = first;
-            child[count++] = first + 1;
+            put(open, first);
+            put(count++, first + 1);
         }
         WideNode n{};
         float far_corner[3];
