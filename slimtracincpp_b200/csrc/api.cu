@@ -196,7 +196,7 @@ struct Context {
     DevArray<float4> d_geometries, d_scene_nodes, d_mesh_nodes, d_tri_hot, d_tri_cold;
     DevArray<WideNode> d_wide_nodes;
     DevArray<WideLeaf> d_wide_leaves;
-    DevArray<SlimMaterial> d_materials;
+    DevArray<float4> d_materials;
     DevArray<float4> d_lights;
     DevArray<uint32_t> d_leaf_geometry, d_emissive_quads, d_refit_order;
     DevArray<DevMesh> d_meshes;
@@ -469,6 +469,20 @@ int upload_geometries(Context &c, const SlimSceneData *s) {
     return upload_emissive(c);
 }
 
+// Material record: the reference's 68 bytes as whole 16-byte words.
+void pack_material(const SlimMaterial &m, std::vector<float4> &out) {
+    const uint32_t bits = (uint32_t)m.flags | (uint32_t)m.texture_count << 8 | (uint32_t)m.texture_ids[0] << 16 |
+                          (uint32_t)m.texture_ids[1] << 24;
+    float packed, brdf;
+    memcpy(&packed, &bits, 4);
+    memcpy(&brdf, &m.brdf, 4);
+    out.push_back(make_float4(m.albedo[0], m.albedo[1], m.albedo[2], m.roughness));
+    out.push_back(make_float4(m.emission[0], m.emission[1], m.emission[2], m.IOR));
+    out.push_back(make_float4(m.reflectivity[0], m.reflectivity[1], m.reflectivity[2], m.metalness));
+    out.push_back(make_float4(m.uv_repeat.x, m.uv_repeat.y, m.normal_magnitude, packed));
+    out.push_back(make_float4(brdf, 0.0f, 0.0f, 0.0f));
+}
+
 int upload_materials(Context &c, const SlimSceneData *s) {
     uint32_t n = c.counts.materials;
     for (uint32_t m = 0; m < n; m++) {
@@ -478,9 +492,11 @@ int upload_materials(Context &c, const SlimSceneData *s) {
                 return set_error(SLIM_ERR_ARGUMENT, "material texture id out of range");
     }
     c.materials.assign(s->materials, s->materials + n);
-    int rc = c.d_materials.reserve(n, "alloc materials");
+    int rc = c.d_materials.reserve(5 * (size_t)n, "alloc materials");
     if (rc) return rc;
-    SLIM_CUDA(cudaMemcpy(c.d_materials.ptr, s->materials, n * sizeof(SlimMaterial), cudaMemcpyHostToDevice), "upload materials");
+    std::vector<float4> packed;
+    for (uint32_t m = 0; m < n; m++) pack_material(s->materials[m], packed);
+    SLIM_CUDA(cudaMemcpy(c.d_materials.ptr, packed.data(), packed.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload materials");
     c.scene.materials = c.d_materials.ptr;
     return c.geometries.empty() ? SLIM_OK : upload_emissive(c);
 }
@@ -1943,7 +1959,7 @@ struct BatchState {
     std::vector<DevScene> h_scenes;
     std::vector<DevFrame> h_frames;
     DevArray<float4> geometries, scene_nodes;
-    DevArray<SlimMaterial> materials;
+    DevArray<float4> materials;
     DevArray<float4> lights;
     DevArray<uint32_t> leaf_geometry, emissive;
     DevArray<DevScene> scenes;
@@ -2253,7 +2269,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
     }
     int rc;
     if ((rc = b.geometries.reserve(4 * n_geo, "alloc batch geometries"))) return rc;
-    if ((rc = b.materials.reserve(n_mat, "alloc batch materials"))) return rc;
+    if ((rc = b.materials.reserve(5 * n_mat, "alloc batch materials"))) return rc;
     if ((rc = b.lights.reserve(n_light ? 3 * n_light : 1, "alloc batch lights"))) return rc;
     if ((rc = b.scene_nodes.reserve(2 * n_node, "alloc batch scene BVHs"))) return rc;
     if ((rc = b.leaf_geometry.reserve(n_geo, "alloc batch leaf indices"))) return rc;
@@ -2261,11 +2277,11 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
     if ((rc = b.scenes.reserve(count, "alloc batch scene table"))) return rc;
     if ((rc = b.frames.reserve(count, "alloc batch frame table"))) return rc;
     std::vector<float4> geo(4 * n_geo);
-    std::vector<SlimMaterial> mat;
+    std::vector<float4> mat;
     std::vector<float4> lig;
     std::vector<SlimBVHNode> nodes;
     std::vector<uint32_t> leaf, emis;
-    mat.reserve(n_mat);
+    mat.reserve(5 * n_mat);
     lig.reserve(3 * n_light);
     nodes.reserve(n_node);
     leaf.reserve(n_geo);
@@ -2302,7 +2318,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         }
         S.emissive_quad_count = emissive;
         og += s->counts.geometries;
-        mat.insert(mat.end(), s->materials, s->materials + s->counts.materials);
+        for (uint32_t m = 0; m < s->counts.materials; m++) pack_material(s->materials[m], mat);
         for (uint32_t l = 0; l < s->counts.lights; l++) pack_light(s->lights[l], lig);
         nodes.insert(nodes.end(), s->bvh.nodes, s->bvh.nodes + s->bvh.node_count);
         leaf.insert(leaf.end(), s->bvh_leaf_geometry_indices, s->bvh_leaf_geometry_indices + s->counts.geometries);
@@ -2328,7 +2344,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         b.any_cache |= F.cache_depth != 0;
     }
     SLIM_CUDA(cudaMemcpy(b.geometries.ptr, geo.data(), geo.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload batch geometries");
-    SLIM_CUDA(cudaMemcpy(b.materials.ptr, mat.data(), mat.size() * sizeof(SlimMaterial), cudaMemcpyHostToDevice), "upload batch materials");
+    SLIM_CUDA(cudaMemcpy(b.materials.ptr, mat.data(), mat.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload batch materials");
     if (!lig.empty())
         SLIM_CUDA(cudaMemcpy(b.lights.ptr, lig.data(), lig.size() * sizeof(float4), cudaMemcpyHostToDevice), "upload batch lights");
     SLIM_CUDA(cudaMemcpy(b.scene_nodes.ptr, nodes.data(), nodes.size() * sizeof(SlimBVHNode), cudaMemcpyHostToDevice), "upload batch BVHs");

@@ -5,6 +5,8 @@
 //   geometry       4 x float4   rotation quat | position,type | scale,material | 1/scale,flags+mesh
 //   BVH node       2 x float4   the reference's 32-byte BVHNode bytes unchanged
 //                               (min.xyz, max.x | max.yz, first_index, leaf_count/depth/flags)
+//   material       5 x float4   albedo, roughness | emission, IOR | reflectivity, metalness | uv repeat, normal
+//                               magnitude, flags+textures | brdf
 //   light          3 x float4   position or direction, intensity | colour, flags | 64/intensity, intensity/64
 //   wide node      5 x uint4    four children's boxes, for the persistent mesh walks (wide_bvh.h)
 //   wide leaf      8 x float4   a leaf's BVH node and the hot bytes of its first two triangles
@@ -56,7 +58,7 @@ struct DevTexture {
 
 struct DevScene {
     const float4 *geometries;      // 4 float4 per geometry
-    const SlimMaterial *materials;
+    const float4 *materials;       // 5 float4 per material
     const float4 *lights;          // 3 float4 per light
     const float4 *scene_nodes;     // 2 float4 per node
     const uint32_t *leaf_geometry; // bvh_leaf_geometry_indices

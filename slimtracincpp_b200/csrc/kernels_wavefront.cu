@@ -1364,13 +1364,11 @@ SLIM_D void append_query(const CacheArgs &C, uint32_t q, const float4 f[4], floa
 }
 
 // ---- shade: colour of this segment, next bounce, finished paths --------
-// Capped at 80 registers (3 blocks per SM instead of 2): latency-bound, the
-// extra warps pay for the spills (config 2: shade 0.180 -> 0.173 ms).  The
-// spills are real traffic -- in round 1, 340 MB of local stores reach L2
-// (ncu) -- but on the final build 2 blocks at 128 registers, without
-// spills, measure the same (0.183 against 0.182 ms).
+// Capped at 64 registers (4 blocks per SM): latency-bound, the extra warps pay
+// for the spills (mesh 1080p 1.138 ms, textures 1080p 393 us; 3 blocks at 80
+// registers 1.143 and 400; 2 at 128 1.146 and 406).
 #ifndef SLIM_SHADE_BLOCKS
-#define SLIM_SHADE_BLOCKS 3
+#define SLIM_SHADE_BLOCKS 4
 #endif
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(256, SLIM_SHADE_BLOCKS) k_shade(DevScene S0, DevFrame F0, QueueArgs A) {

@@ -766,23 +766,24 @@ struct Mat {
     float3 reflectivity; float metalness;
 };
 SLIM_D Mat load_mat(const DevScene &S, uint32_t i) {
-    const SlimMaterial *p = S.materials + i;
+    const float4 *p = S.materials + 5 * (size_t)i;
+    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
     Mat m;
-    m.albedo = ld3(p->albedo);
-    m.roughness = __ldg(&p->roughness);
-    uint32_t packed = __ldg(reinterpret_cast<const uint32_t *>(&p->flags));
+    m.albedo = xyz(a);
+    m.roughness = a.w;
+    m.emission = xyz(b);
+    m.IOR = b.w;
+    m.reflectivity = xyz(c);
+    m.metalness = c.w;
+    m.rep_u = d.x;
+    m.rep_v = d.y;
+    m.normal_magnitude = d.z;
+    const uint32_t packed = __float_as_uint(d.w);
     m.flags = packed & 0xFFu;
     m.texture_count = (packed >> 8) & 0xFFu;
     m.tex0 = (packed >> 16) & 0xFFu;
     m.tex1 = packed >> 24;
-    m.brdf = __ldg(&p->brdf);
-    m.normal_magnitude = __ldg(&p->normal_magnitude);
-    m.rep_u = __ldg(&p->uv_repeat.x);
-    m.rep_v = __ldg(&p->uv_repeat.y);
-    m.emission = ld3(p->emission);
-    m.IOR = __ldg(&p->IOR);
-    m.reflectivity = ld3(p->reflectivity);
-    m.metalness = __ldg(&p->metalness);
+    m.brdf = __float_as_int(__ldg(&p[4].x));
     return m;
 }
 // Small whole powers, rounded once: the products carry their rounding errors
