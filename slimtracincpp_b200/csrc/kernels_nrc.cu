@@ -71,7 +71,18 @@ SLIM_N uint32_t pack2(float a, float b) {
 SLIM_N float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 SLIM_N float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
+// max(0, x) of both halves (NaN: 0): the same as before the rounding, in half
+// the instructions (1,036,801 queries 102.5 -> 96.6 us).
+SLIM_N uint32_t relu2(uint32_t w) {
+    uint32_t r;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0u));
+    return r;
+}
+
 // Row r, column group g (8 values) of a 128-row image.
+SLIM_N void store_row(uint8_t *img, uint32_t r, uint32_t g, uint4 q) {
+    *(uint4 *)(img + g * (kTile * 16u) + r * 16u) = q;
+}
 SLIM_N void store8(uint8_t *img, uint32_t r, uint32_t g, const float v[8]) {
     uint4 q = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
     *(uint4 *)(img + g * (kTile * 16u) + r * 16u) = q;
@@ -171,10 +182,9 @@ SLIM_N void epilogue_relu(uint32_t lane_addr, uint8_t *H, uint32_t r) {
         tmem_ld32(lane_addr + 32u * half, v);
 #pragma unroll
         for (int g = 0; g < 4; g++) {
-            float w[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) w[j] = fmaxf(v[8 * g + j], 0.0f);
-            store8(H, r, 4 * half + g, w);
+            const float *w = v + 8 * g;
+            store_row(H, r, 4 * half + g, make_uint4(relu2(pack2(w[0], w[1])), relu2(pack2(w[2], w[3])),
+                                                      relu2(pack2(w[4], w[5])), relu2(pack2(w[6], w[7]))));
         }
     }
 }
@@ -218,7 +228,9 @@ SLIM_N void sync_for_mma() {
 // input rows, which are dead after the first layer, and all its layers share
 // 64 TMEM columns: 24 KB of shared memory and an eighth of the columns a tile.
 // 1,036,801 samples: 196 us with two tiles per SM, 149 us with six, 102 us with
-// packed conversions (pack2) besides.
+// packed conversions (pack2) besides, 97 us with packed ReLUs (relu2).  It now
+// issues in 56 % of the cycles (73.7 M warp instructions before relu2), more
+// than half of that for the 36 sincospif of a sample.
 constexpr uint32_t kGroups = 3;
 SLIM_N void group_sync(uint32_t group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory"); }
 SLIM_N void group_sync_for_mma(uint32_t group) {
