@@ -317,8 +317,8 @@ int slimRenderToDevice(const SlimCanvasData *canvas, const SlimCameraRayProjecti
  * thread captures a CUDA graph in global capture mode, which makes
  * cudaMalloc/cudaFree fail process-wide, or inside a host engine that
  * reserves all device memory up front.  The queues live in one file-scope
- * __device__ array of 64 MiB (and 16 KiB of counters) that every GPU loading the library holds until
- * exit; frames needing more (about 250 bytes per sample, e.g. 640x360 with
+ * __device__ array of 64 MiB (and 16 KiB of counters) that every GPU loading
+ * the library holds until exit; frames needing more (about 250 bytes per sample, e.g. 640x360 with
  * several lights fits, 1080p does not) fail with SLIM_ERR_LIMIT.  The first
  * call on each device looks up the array's device address
  * (cudaGetSymbolAddress), so make that first call before any stream

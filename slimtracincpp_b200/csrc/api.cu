@@ -1638,7 +1638,7 @@ int noalloc_layout(unsigned char *base, uint32_t samples, uint32_t lights, Wavef
     B.rays[1] = (float4 *)take(32 * n);
     B.hits = (float4 *)take(48 * n);
     B.shadow_mask = (unsigned long long *)take(8 * n);
-    take(8 * sizeof(uint32_t));
+    take(8 * sizeof(uint32_t));    // unused: the frames that fit are those that did with the counters here
     B.queue_count = (uint32_t *)(base + kNoAllocScratchBytes);
     if (off > kNoAllocScratchBytes) return set_error(SLIM_ERR_LIMIT, "frame larger than the no-alloc scratch (64 MiB)");
     size_t left = kNoAllocScratchBytes - off;

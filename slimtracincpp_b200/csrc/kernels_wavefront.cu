@@ -36,8 +36,6 @@ namespace dev {
 
 SLIM_D uint32_t lane_id() { return threadIdx.x & 31u; }
 
-
-
 // Warp-aggregated queue append: one atomicAdd per warp, slots handed out
 // by the ballot's prefix popcount.  Returns the slot of a thread whose
 // `want` is set.
