@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cmath>
 #include <condition_variable>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -208,6 +209,7 @@ struct Context {
     DevArray<uint32_t> d_error;
     DevArray<unsigned long long> d_counters;
     std::vector<uint32_t> refit_order;
+    LeafList leaf_list{};                 // as uploaded, but for refitted boxes
     std::vector<LeafRange> leaf_ranges;   // of the listed scene leaves, and the geometries they name
     std::vector<uint32_t> leaf_geometry;
     uint32_t scene_node_count = 0;
@@ -416,12 +418,15 @@ int upload_emissive(Context &c) {
     return SLIM_OK;
 }
 
-// The leaves of a scene BVH small enough to test one by one (see DevScene),
+constexpr uint32_t kMostListedNodes = 2 * kMaxListedLeaves + 64;      // unreachable nodes among them
+static_assert(kMostListedNodes <= 256, "LeafList::node holds a byte");
+
+// The leaves of a scene BVH small enough to test one by one (see LeafList),
 // and [first, end) of the leaf geometry indices for each.
-void list_leaves(DevScene &S, const SlimBVHNode *nodes, uint32_t node_count, std::vector<LeafRange> &ranges) {
-    S.listed_leaves = 0;
+void list_leaves(LeafList &L, const SlimBVHNode *nodes, uint32_t node_count, std::vector<LeafRange> &ranges) {
+    L = LeafList{};
     ranges.clear();
-    if (nodes[0].leaf_count || node_count > 2 * kMaxListedLeaves + 64 || !boxes_nest(nodes, node_count)) return;
+    if (nodes[0].leaf_count || node_count > kMostListedNodes || !boxes_nest(nodes, node_count)) return;
     std::vector<uint8_t> reached(node_count, 0);
     reached[0] = 1;
     for (uint32_t i = 0; i < node_count; i++) {
@@ -430,23 +435,24 @@ void list_leaves(DevScene &S, const SlimBVHNode *nodes, uint32_t node_count, std
             reached[nodes[i].first_index] = reached[nodes[i].first_index + 1] = 1;
             continue;
         }
-        if (ranges.size() == kMaxListedLeaves || i > 255) {
+        if (ranges.size() == kMaxListedLeaves) {
             ranges.clear();
             return;
         }
-        S.leaf_node[ranges.size()] = (uint8_t)i;
+        L.node[ranges.size()] = (uint8_t)i;
+        L.leaf[ranges.size()] = nodes[i];
         ranges.push_back({nodes[i].first_index, nodes[i].first_index + nodes[i].leaf_count});
     }
-    S.listed_leaves = (uint32_t)ranges.size();
+    L.count = (uint32_t)ranges.size();
 }
-void sort_leaves(DevScene &S, const std::vector<LeafRange> &ranges, const uint32_t *leaf_geometry,
+void sort_leaves(LeafList &L, const std::vector<LeafRange> &ranges, const uint32_t *leaf_geometry,
                  const SlimGeometry *geometries) {
-    S.implicit_leaves = S.mesh_leaves = S.shadow_leaves = 0;
+    L.implicit_leaves = L.mesh_leaves = L.shadow_leaves = 0;
     for (uint32_t j = 0; j < ranges.size(); j++)
         for (uint32_t k = ranges[j].first; k < ranges[j].end; k++) {
             const SlimGeometry &g = geometries[leaf_geometry[k]];
-            if (g.flags & SLIM_GEOMETRY_IS_VISIBLE) (g.type == SLIM_GEOMETRY_MESH ? S.mesh_leaves : S.implicit_leaves) |= 1u << j;
-            if (g.flags & SLIM_GEOMETRY_IS_SHADOWING) S.shadow_leaves |= 1u << j;
+            if (g.flags & SLIM_GEOMETRY_IS_VISIBLE) (g.type == SLIM_GEOMETRY_MESH ? L.mesh_leaves : L.implicit_leaves) |= 1u << j;
+            if (g.flags & SLIM_GEOMETRY_IS_SHADOWING) L.shadow_leaves |= 1u << j;
         }
 }
 
@@ -465,7 +471,16 @@ int upload_geometries(Context &c, const SlimSceneData *s) {
     SLIM_CUDA(cudaMemcpy(c.d_geometries.ptr, packed.data(), packed.size() * sizeof(float4), cudaMemcpyHostToDevice),
               "upload geometries");
     c.scene.geometries = c.d_geometries.ptr;
-    if (c.leaf_geometry.size() == n) sort_leaves(c.scene, c.leaf_ranges, c.leaf_geometry.data(), c.geometries.data());
+    if (c.leaf_list.count && c.leaf_geometry.size() == n) {
+        LeafList list = c.leaf_list;
+        sort_leaves(list, c.leaf_ranges, c.leaf_geometry.data(), c.geometries.data());
+        // its first words; objects that only move keep them
+        const size_t head = offsetof(LeafList, node);
+        if (memcmp(&list, &c.leaf_list, head)) {
+            SLIM_CUDA(cudaMemcpy(c.d_scene_nodes.ptr, &list, head, cudaMemcpyHostToDevice), "upload leaf list");
+            c.leaf_list = list;
+        }
+    }
     return upload_emissive(c);
 }
 
@@ -540,11 +555,23 @@ int upload_scene_bvh(Context &c, const SlimSceneData *s) {
     if (bvh_depth(s->bvh.nodes, n) + 2 > (uint32_t)kStackCapacity) return set_error(SLIM_ERR_LIMIT, "scene BVH deeper than the traversal stack");
     for (uint32_t g = 0; g < c.counts.geometries; g++)
         if (s->bvh_leaf_geometry_indices[g] >= c.counts.geometries) return set_error(SLIM_ERR_ARGUMENT, "scene BVH leaf index out of range");
-    rc = c.d_scene_nodes.reserve(2 * (size_t)n, "alloc scene BVH");
+    rc = c.d_scene_nodes.reserve(2 * (kLeafListNodes + (size_t)n), "alloc scene BVH");
     if (rc) return rc;
     rc = c.d_leaf_geometry.reserve(c.counts.geometries, "alloc leaf indices");
     if (rc) return rc;
-    SLIM_CUDA(cudaMemcpy(c.d_scene_nodes.ptr, s->bvh.nodes, n * sizeof(SlimBVHNode), cudaMemcpyHostToDevice), "upload scene BVH");
+    list_leaves(c.leaf_list, s->bvh.nodes, n, c.leaf_ranges);
+    c.leaf_geometry.assign(s->bvh_leaf_geometry_indices, s->bvh_leaf_geometry_indices + c.counts.geometries);
+    sort_leaves(c.leaf_list, c.leaf_ranges, c.leaf_geometry.data(), c.geometries.data());
+    // the leaf list, then the nodes: those of a small scene in one copy
+    const uint32_t joined = std::min(n, kMostListedNodes);
+    SlimBVHNode head[kLeafListNodes + kMostListedNodes];
+    memcpy(head, &c.leaf_list, sizeof(LeafList));
+    memcpy(head + kLeafListNodes, s->bvh.nodes, joined * sizeof(SlimBVHNode));
+    SLIM_CUDA(cudaMemcpy(c.d_scene_nodes.ptr, head, (kLeafListNodes + joined) * sizeof(SlimBVHNode),
+                         cudaMemcpyHostToDevice), "upload scene BVH");
+    if (n > joined)
+        SLIM_CUDA(cudaMemcpy(c.d_scene_nodes.ptr + 2 * (kLeafListNodes + joined), s->bvh.nodes + joined,
+                             (n - joined) * sizeof(SlimBVHNode), cudaMemcpyHostToDevice), "upload scene BVH");
     SLIM_CUDA(cudaMemcpy(c.d_leaf_geometry.ptr, s->bvh_leaf_geometry_indices, c.counts.geometries * 4, cudaMemcpyHostToDevice),
               "upload leaf indices");
     build_refit_order(c, s->bvh.nodes, n);
@@ -554,13 +581,11 @@ int upload_scene_bvh(Context &c, const SlimSceneData *s) {
         SLIM_CUDA(cudaMemcpy(c.d_refit_order.ptr, c.refit_order.data(), c.refit_order.size() * 4, cudaMemcpyHostToDevice),
                   "upload refit order");
     c.scene_node_count = n;
-    c.scene.scene_nodes = c.d_scene_nodes.ptr;
+    c.scene.leaves = reinterpret_cast<const LeafList *>(c.d_scene_nodes.ptr);
+    c.scene.scene_nodes = c.d_scene_nodes.ptr + 2 * kLeafListNodes;
     c.scene.leaf_geometry = c.d_leaf_geometry.ptr;
     c.scene.scene_node_count = n;
     c.scene.flags = s->flags;
-    list_leaves(c.scene, s->bvh.nodes, n, c.leaf_ranges);
-    c.leaf_geometry.assign(s->bvh_leaf_geometry_indices, s->bvh_leaf_geometry_indices + c.counts.geometries);
-    sort_leaves(c.scene, c.leaf_ranges, c.leaf_geometry.data(), c.geometries.data());
     return SLIM_OK;
 }
 
@@ -1292,6 +1317,7 @@ int slimInitDataOnGPU(const SlimSceneData *scene) {
     c.counts = scene->counts;
     c.geometries.clear();
     c.materials.clear();
+    c.leaf_list = LeafList{};
     c.leaf_geometry.clear();
     c.leaf_ranges.clear();
     if ((rc = upload_materials(c, scene))) return rc;
@@ -1490,7 +1516,7 @@ int slimDownloadSceneBVH(SlimSceneData *scene) {
     if (scene->bvh.node_count != c.scene_node_count)
         return set_error(SLIM_ERR_STATE, "scene BVH node count differs from the uploaded one");
     if (c.refit_done) SLIM_CUDA(cudaEventSynchronize(c.refit_done), "wait for the refit");
-    SLIM_CUDA(cudaMemcpy(scene->bvh.nodes, c.d_scene_nodes.ptr, c.scene_node_count * sizeof(SlimBVHNode),
+    SLIM_CUDA(cudaMemcpy(scene->bvh.nodes, c.scene.scene_nodes, c.scene_node_count * sizeof(SlimBVHNode),
                          cudaMemcpyDeviceToHost), "download scene BVH");
     return SLIM_OK;
 }
@@ -1499,7 +1525,8 @@ int slimRefitSceneBVH(void *stream) {
     std::lock_guard<std::mutex> lock(g_mutex);
     Context &c = g_ctx;
     if (!c.initialized) return set_error(SLIM_ERR_STATE, "slimInitDataOnGPU has not been called");
-    cudaError_t e = launch_refit_scene_bvh(c.scene, c.d_scene_nodes.ptr, c.d_refit_order.ptr,
+    cudaError_t e = launch_refit_scene_bvh(c.scene, c.d_scene_nodes.ptr + 2 * kLeafListNodes,
+                                           reinterpret_cast<LeafList *>(c.d_scene_nodes.ptr), c.d_refit_order.ptr,
                                            (uint32_t)c.refit_order.size(), (cudaStream_t)stream, timer_for(c));
     if (e != cudaSuccess) return cuda_fail(e, "refit launch");
     // the next frame, on whatever stream, reads the refit nodes
@@ -2265,7 +2292,7 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         n_geo += s->counts.geometries;
         n_mat += s->counts.materials;
         n_light += s->counts.lights;
-        n_node += s->bvh.node_count;
+        n_node += kLeafListNodes + s->bvh.node_count;
     }
     int rc;
     if ((rc = b.geometries.reserve(4 * n_geo, "alloc batch geometries"))) return rc;
@@ -2295,7 +2322,8 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         S.geometries = b.geometries.ptr + 4 * og;
         S.materials = b.materials.ptr + mat.size();
         S.lights = b.lights.ptr + lig.size();
-        S.scene_nodes = b.scene_nodes.ptr + 2 * nodes.size();
+        S.leaves = reinterpret_cast<const LeafList *>(b.scene_nodes.ptr + 2 * nodes.size());
+        S.scene_nodes = b.scene_nodes.ptr + 2 * (nodes.size() + kLeafListNodes);
         S.leaf_geometry = b.leaf_geometry.ptr + leaf.size();
         S.emissive_quads = b.emissive.ptr + emis.size();
         S.geometry_count = s->counts.geometries;
@@ -2303,9 +2331,12 @@ int slimBatchSetRequests(const SlimRenderRequest *requests, uint32_t count) {
         S.light_count = s->counts.lights;
         S.scene_node_count = s->bvh.node_count;
         S.flags = s->flags;
+        LeafList list;
         std::vector<LeafRange> ranges;
-        list_leaves(S, s->bvh.nodes, s->bvh.node_count, ranges);
-        sort_leaves(S, ranges, s->bvh_leaf_geometry_indices, s->geometries);
+        list_leaves(list, s->bvh.nodes, s->bvh.node_count, ranges);
+        sort_leaves(list, ranges, s->bvh_leaf_geometry_indices, s->geometries);
+        const SlimBVHNode *list_words = reinterpret_cast<const SlimBVHNode *>(&list);
+        nodes.insert(nodes.end(), list_words, list_words + kLeafListNodes);
         uint32_t emissive = 0, instances = 0;
         for (uint32_t g = 0; g < s->counts.geometries; g++) {
             const SlimGeometry &G = s->geometries[g];

@@ -56,6 +56,24 @@ struct DevTexture {
     uint32_t _pad[3];
 };
 
+// The leaves of a small scene BVH, for rays that test every leaf's box instead
+// of walking the tree.  It lies in device memory in front of the nodes and is
+// written by the uploads and the refit that write them, so a frame captured
+// into a graph follows these.
+constexpr uint32_t kMaxListedLeaves = 32;
+struct alignas(128) LeafList {
+    // 0: more leaves than kMaxListedLeaves, a root leaf, or boxes that do not nest
+    uint32_t count;
+    // of them, those with a visible implicit primitive, a visible mesh
+    // instance, anything that casts shadows
+    uint32_t implicit_leaves, mesh_leaves, shadow_leaves;
+    uint8_t node[kMaxListedLeaves];             // their node indices
+    uint32_t _pad[20];
+    SlimBVHNode leaf[kMaxListedLeaves];         // their nodes
+};
+static_assert(sizeof(LeafList) == 1152, "LeafList is nine cache lines");
+constexpr uint32_t kLeafListNodes = sizeof(LeafList) / sizeof(SlimBVHNode);
+
 struct DevScene {
     const float4 *geometries;      // 4 float4 per geometry
     const float4 *materials;       // 5 float4 per material
@@ -76,16 +94,8 @@ struct DevScene {
     uint32_t emissive_quad_count;
     uint32_t flags;                // SLIM_SCENE_HAD_EMISSIVE_QUADS
     uint32_t scene_node_count;
-    // Leaves of a small scene BVH (node indices; count 0: larger than
-    // kMaxListedLeaves, a root leaf, or boxes that do not nest), for rays that
-    // test every leaf's box instead of walking the tree.
-    uint32_t listed_leaves;
-    // of them, those with a visible implicit primitive, a visible mesh
-    // instance, anything that casts shadows
-    uint32_t implicit_leaves, mesh_leaves, shadow_leaves;
-    uint8_t leaf_node[32];
+    const LeafList *leaves;
 };
-constexpr uint32_t kMaxListedLeaves = 32;
 
 // Per-frame parameters of a render launch.
 struct DevFrame {

@@ -194,9 +194,11 @@ cudaError_t launch_batch_persistent(const DevScene *scenes, const DevFrame *fram
                                     uint32_t *error_flags, unsigned long long *counters, cudaStream_t stream);
 
 // GPU refit of the scene BVH: recomputes every node's bounds bottom-up from
-// the geometries' world AABBs, keeping the uploaded topology.
-cudaError_t launch_refit_scene_bvh(const DevScene &S, float4 *scene_nodes, const uint32_t *parent_order,
-                                   uint32_t node_count, cudaStream_t stream, StageTimer *timer);
+// the geometries' world AABBs, keeping the uploaded topology, and the listed
+// leaves' copies.
+cudaError_t launch_refit_scene_bvh(const DevScene &S, float4 *scene_nodes, LeafList *list,
+                                   const uint32_t *parent_order, uint32_t node_count, cudaStream_t stream,
+                                   StageTimer *timer);
 
 // bmp2texture's texel-quad baker on the device (kernels_bake.cu): the
 // arguments and results of slimBakeTexture, on `stream`, synchronous.

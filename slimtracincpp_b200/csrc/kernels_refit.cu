@@ -79,12 +79,20 @@ __global__ void k_refit_inner(float4 *nodes, const uint32_t *order, uint32_t cou
     if (threadIdx.x == 0 && blockIdx.x == 0) refit_inner(nodes, order, count);
 }
 
-// Scenes of up to kRefitBlock nodes: both passes in one block, one launch.
+// Scenes of up to kRefitBlock nodes, listed leaves among them: both passes in
+// one block, one launch.
 constexpr uint32_t kRefitBlock = 1024;
 __global__ void __launch_bounds__(kRefitBlock) k_refit_small(DevScene S, float4 *nodes, uint32_t node_count,
-                                                             const uint32_t *order, uint32_t inner_count) {
+                                                             const uint32_t *order, uint32_t inner_count,
+                                                             LeafList *list) {
     if (threadIdx.x < node_count) refit_leaf(S, nodes, threadIdx.x);
     __syncthreads();
+    for (uint32_t j = threadIdx.x; j < list->count; j += blockDim.x) {      // the listed leaves' copies
+        float4 *leaf = reinterpret_cast<float4 *>(list->leaf + j);
+        const float4 *node = nodes + 2 * (uint32_t)list->node[j];
+        leaf[0] = node[0];
+        leaf[1] = node[1];
+    }
     if (threadIdx.x == 0) {
         __threadfence_block();
         refit_inner(nodes, order, inner_count);
@@ -93,14 +101,14 @@ __global__ void __launch_bounds__(kRefitBlock) k_refit_small(DevScene S, float4 
 
 }  // namespace dev
 
-cudaError_t launch_refit_scene_bvh(const DevScene &S, float4 *scene_nodes, const uint32_t *order, uint32_t inner_count,
-                                   cudaStream_t stream, StageTimer *timer) {
+cudaError_t launch_refit_scene_bvh(const DevScene &S, float4 *scene_nodes, LeafList *list, const uint32_t *order,
+                                   uint32_t inner_count, cudaStream_t stream, StageTimer *timer) {
     uint32_t n = S.scene_node_count;
     if (!n) return cudaSuccess;
     if (timer) timer->begin(STAGE_REFIT, stream);
     if (n <= dev::kRefitBlock) {
         const uint32_t threads = (n + 31) / 32 * 32;
-        dev::k_refit_small<<<1, threads, 0, stream>>>(S, scene_nodes, n, order, inner_count);
+        dev::k_refit_small<<<1, threads, 0, stream>>>(S, scene_nodes, n, order, inner_count, list);
         count_launch();
         if (timer) timer->end(STAGE_REFIT, stream);
         return cudaGetLastError();

@@ -404,9 +404,10 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
         bool occluded = false;
         float ln, rn, lf, rf;
         float4 ra, rb;
-        if (!COUNT && S.listed_leaves && finite_ray(ray)) {
-            for (uint32_t leaves = leaves_hit(S, ray, Ld, S.shadow_leaves); leaves && !occluded; leaves &= leaves - 1u) {
-                load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], ra, rb);
+        const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
+        if (!COUNT && list.x && finite_ray(ray)) {
+            for (uint32_t leaves = leaves_hit(S, list.x, ray, Ld, list.w); leaves && !occluded; leaves &= leaves - 1u) {
+                load_leaf(S, __ffs((int)leaves) - 1, ra, rb);
                 hit_box_finite(ray, ra, rb, ln, lf);
                 occluded = shadow_leaf<COUNT>(S, A, tag, node_first(rb), node_leaf_count(rb), lf, ray, Ld, mesh_stack,
                                               err, w);
@@ -853,15 +854,15 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
         // known.  Candidates are numbered in that order from 1; an implicit hit
         // has 0, and a candidate at exactly the ray's best distance that is not
         // its holder sends the ray to the whole walk (k_extend_resolve).
-        bool listed = !COUNT && S.listed_leaves && finite_ray(r);
-        if (listed) {
-            const uint32_t leaves = leaves_hit(S, r, INFINITY, S.implicit_leaves | S.mesh_leaves);
+        const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
+        if (!COUNT && list.x && finite_ray(r)) {
+            const uint32_t leaves = leaves_hit(S, list.x, r, INFINITY, list.y | list.z);
             Nearest seen;
-            best_geo = closest_of_leaves<COUNT>(S, leaves & S.implicit_leaves, r, hit, seen, err, w);
-            for (uint32_t rest = leaves & S.mesh_leaves; rest && !seen.unsure; rest &= rest - 1u) {
+            best_geo = closest_of_leaves<COUNT>(S, leaves & list.y, r, hit, seen, err, w);
+            for (uint32_t rest = leaves & list.z; rest && !seen.unsure; rest &= rest - 1u) {
                 float4 a, b;
                 float ln, lf;
-                load_node(S.scene_nodes, S.leaf_node[__ffs((int)rest) - 1], a, b);
+                load_leaf(S, __ffs((int)rest) - 1, a, b);
                 hit_box_finite(r, a, b, ln, lf);
                 if (ln > hit.distance * kReachSlack) continue;
                 const uint32_t first = node_first(b), count = node_leaf_count(b);

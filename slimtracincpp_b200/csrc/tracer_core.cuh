@@ -541,19 +541,26 @@ SLIM_D int hit_geometries(const DevScene &S, uint32_t first, uint32_t count, flo
     return hit_geo;
 }
 
-// The leaves `of` a small scene whose boxes the ray hits before `reach`: bit j
-// is leaf S.leaf_node[j].  Every box is tested: leaving out those not asked
-// for costs more in the loop than it saves (implicit scenes 95 against 89 us).
+// The first words of a scene's leaf list: how many, which hold visible implicit
+// primitives, visible mesh instances, anything that casts shadows.
+SLIM_D uint4 listed_leaves(const DevScene &S) { return __ldg(reinterpret_cast<const uint4 *>(S.leaves)); }
+SLIM_D void load_leaf(const DevScene &S, uint32_t j, float4 &a, float4 &b) {
+    load_node(reinterpret_cast<const float4 *>(S.leaves->leaf), j, a, b);
+}
+
+// The leaves `of` a small scene's `count` whose boxes the ray hits before
+// `reach`.  Every box is tested: leaving out those not asked for costs more in
+// the loop than it saves (implicit scenes 95 against 89 us).
 // A leaf's box lies in the boxes above it, so the
 // tree walk reaches the same leaves; the loop has no stack, no waiting loads
 // and no divergence.
-SLIM_D uint32_t leaves_hit(const DevScene &S, const Ray &r, float reach, uint32_t of) {
+SLIM_D uint32_t leaves_hit(const DevScene &S, uint32_t count, const Ray &r, float reach, uint32_t of) {
     uint32_t hit = 0;
 #pragma unroll 4
-    for (uint32_t j = 0; j < S.listed_leaves; j++) {
+    for (uint32_t j = 0; j < count; j++) {
         float4 a, b;
         float near, far;
-        load_node(S.scene_nodes, S.leaf_node[j], a, b);
+        load_leaf(S, j, a, b);
         if (hit_box_finite(r, a, b, near, far) && near < reach) hit |= 1u << j;
     }
     return hit & of;
@@ -594,7 +601,7 @@ SLIM_D int closest_of_leaves(const DevScene &S, uint32_t leaves, const Ray &r, H
     while (leaves) {
         float4 a, b;
         float ln, lf;
-        load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], a, b);
+        load_leaf(S, __ffs((int)leaves) - 1, a, b);
         leaves &= leaves - 1u;
         hit_box_finite(r, a, b, ln, lf);
         if (ln > hit.distance * kReachSlack) continue;
@@ -625,13 +632,14 @@ SLIM_D int scene_trace(const DevScene &S, Ray &r, Hit &hit, bool any_hit, float 
                        uint32_t *stack, uint32_t *mesh_stack, uint32_t &err, Work &w) {
     reset(r, scale_add(r.d, kTraceOffset, r.o), r.d);
     hit.distance = max_distance;
-    if (!COUNT && S.listed_leaves && (any_hit || !S.mesh_count) && finite_ray(r)) {
-        uint32_t leaves = leaves_hit(S, r, max_distance, any_hit ? S.shadow_leaves : S.implicit_leaves);
+    const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
+    if (!COUNT && list.x && (any_hit || !S.mesh_count) && finite_ray(r)) {
+        uint32_t leaves = leaves_hit(S, list.x, r, max_distance, any_hit ? list.w : list.y);
         if (any_hit) {
             while (leaves) {
                 float4 a, b;
                 float ln, lf;
-                load_node(S.scene_nodes, S.leaf_node[__ffs((int)leaves) - 1], a, b);
+                load_leaf(S, __ffs((int)leaves) - 1, a, b);
                 leaves &= leaves - 1u;
                 hit_box_finite(r, a, b, ln, lf);
                 const int g = hit_geometries<COUNT>(S, node_first(b), node_leaf_count(b), lf, r, hit, true, mesh_stack, err, w);
