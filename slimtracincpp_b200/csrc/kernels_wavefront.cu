@@ -769,7 +769,7 @@ SLIM_D float key_distance(unsigned long long key) { return __uint_as_float((uint
 constexpr unsigned long long kNoHitKey = (0x7F800000ull << 32) | 0xFFFFFFFFull;
 
 template <bool COUNT, bool BATCH>
-__global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, QueueArgs A) {
+__global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F0, QueueArgs A) {
     chain_wait();
     uint32_t n = queue_size(A);
     uint32_t stack[kStackCapacity];
@@ -807,8 +807,11 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
             float rn, rf;
             load_node(nodes, 0, ra, rb);
             bump<COUNT>(w.mesh_nodes);
-            // the root test with the largest distance the reference could have used
-            if (!(hit_node(local, ra, rb, rn, rf) && rn < clip && rn <= hit.distance)) return;
+            // the root test with the largest distance the reference could have used:
+            // in its order the best implicit hit so far's; out of it a hit just
+            // in front of the root's box may count too
+            const float reach = seen ? seen->reach(hit.distance) * kReachSlack + slab_margin(local) : hit.distance;
+            if (!(hit_node(local, ra, rb, rn, rf) && rn < clip && rn <= reach)) return;
             if (node_leaf_count(rb)) {
                 // a single-leaf mesh (mesh_tracer.h:66-70): its triangles here
                 Hit mh;
@@ -867,7 +870,7 @@ __global__ void __launch_bounds__(256) k_extend_scene(DevScene S0, DevFrame F0, 
                 float ln, lf;
                 load_leaf(S, __ffs((int)rest) - 1, a, b);
                 hit_box_finite(r, a, b, ln, lf);
-                if (ln > hit.distance * kReachSlack) continue;
+                if (ln > seen.reach(hit.distance) * kReachSlack + slab_margin(r)) continue;
                 const uint32_t first = node_first(b), count = node_leaf_count(b);
                 for (uint32_t i = 0; i < count; i++) {
                     const uint32_t gi = __ldg(S.leaf_geometry + first + i);

@@ -565,8 +565,12 @@ SLIM_D uint32_t leaves_hit(const DevScene &S, uint32_t count, const Ray &r, floa
     }
     return hit & of;
 }
-// Boxes up to this factor beyond the best hit are still looked into.
+// Boxes up to this factor beyond the best hit, and the slab test's rounding
+// (as wide_axis has it: each of a near distance's terms is off by 2^-24 of
+// itself, and plane * rcp is at most the distance beyond |so|), are still
+// looked into.
 constexpr float kReachSlack = 1.0f + 0x1p-18f;
+SLIM_D float slab_margin(const Ray &r) { return 0x1p-20f * max3(fabsf(r.so.x), fabsf(r.so.y), fabsf(r.so.z)); }
 
 // What a closest hit has seen so far when geometries are tested in another
 // order than the reference's.  The reference keeps the first of two hits at
@@ -598,13 +602,14 @@ template <bool COUNT>
 SLIM_D int closest_of_leaves(const DevScene &S, uint32_t leaves, const Ray &r, Hit &hit, Nearest &seen, uint32_t &err,
                              Work &w) {
     int best = -1;
+    const float margin = slab_margin(r);
     while (leaves) {
         float4 a, b;
         float ln, lf;
         load_leaf(S, __ffs((int)leaves) - 1, a, b);
         leaves &= leaves - 1u;
         hit_box_finite(r, a, b, ln, lf);
-        if (ln > hit.distance * kReachSlack) continue;
+        if (ln > seen.reach(hit.distance) * kReachSlack + margin) continue;
         const uint32_t first = node_first(b), count = node_leaf_count(b);
         Hit aux;
         for (uint32_t i = 0; i < count; i++) {

@@ -110,7 +110,8 @@ def frame(scene, view, engine):
 
 
 @pytest.mark.parametrize("size", [(49, 37), (513, 385)])
-@pytest.mark.parametrize("far,distance", [((0.0, 0.0, 0.0), 1.0)])
+@pytest.mark.parametrize("far,distance", [((0.0, 0.0, 0.0), 1.0), ((410.0, 130.0, -270.0), 1.0),
+                                          ((410.0, 130.0, -270.0), 0.03)])
 @pytest.mark.parametrize("side", [-1, 1])
 @pytest.mark.parametrize("turned", [False, True])
 @pytest.mark.parametrize("kind", ["coincident", "overlapping", "quad beside", "quad aside", *IN_A_BOX,
