@@ -739,34 +739,45 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
 //                  publish (distance, k) with a 64-bit atomicMin per ray;
 //   extend_resolve the candidate whose (distance, k) is the ray's minimum
 //                  writes the hit record.
-// Cross-candidate culling keeps ties (<=), so the winner is the reference's.
-// Within a mesh the walk visits leaves in another order than the reference,
-// which keeps the first of two hits at the same distance and skips a leaf
-// whose box begins at or beyond the current hit.  A hit beyond its own box's
-// near distance is reached whatever was hit before, so the nearest hit is the
-// reference's unless another lies between it and its box's near distance
-// (rounding can put the near distance behind the hit) or at the same
-// distance: such a ray is traced whole (k_extend_overflow; none of the 2.07 M
-// primary rays of the 1080p mesh frame).
+// The candidates' walks end in any order, and within a mesh the walk visits
+// leaves in another order than the reference, which keeps the first of two hits
+// at the same distance and skips a leaf whose box begins at or beyond the
+// current hit.  A hit beyond the near distances of the boxes above it is reached
+// whatever was hit before, so the nearest hit is the reference's unless another
+// -- of the same walk, of another candidate, or the best implicit one -- lies at
+// the same distance or between it and those near distances (rounding can put
+// these behind the hit).  A hit's key therefore says how far beyond it other
+// hits matter; they are not culled, and such a ray is traced whole
+// (k_extend_overflow; none in the 1080p mesh frames of 2 and 8 bounces).
 // Few walks are shared like the any-hit ones (a loop of its own, without the
 // sharing's cost for large launches, whose ends the other rays' walks cover):
 // a part culls by the ray's published distance and, if its hit is still the
-// ray's nearest when it ends, appends a record of its own; a hit at the ray's
-// distance that is not its holder -- another part's, another candidate's or an
-// implicit one's may be --, or one not beyond its box's near distance, leaves
-// the ray undecided.
+// ray's nearest when it ends, appends a record of its own; one whose hit is not,
+// but in the held hit's reach, leaves the ray undecided, as do parts with hits
+// at the same distance or with a hit that is not beyond its box's near distance.
 // Candidate records (4 float4): (local origin, clip) (local direction, slot)
-// (wide root, triangle offset, plane bound, 0) (geometry, mesh, k, found); a
-// walk that ends with the ray's nearest hit so far overwrites the third with
-// (t, u, v, triangle | behind << 31) and sets `found`.  The ray keys live in the shadow-mask array, which is
-// free until the shadow stage.
+// (wide root, triangle offset, plane bound, 0) (geometry, mesh, k, -near), near
+// being the near distance of the boxes above the mesh; a walk that ends with a
+// hit overwrites the third with (t, u, v, triangle | behind << 31) and the last
+// word with the hit's own near distance, sign clear.  The ray keys live in the
+// shadow-mask array, which is free until the shadow stage.
 
-SLIM_D unsigned long long hit_key(float t, uint32_t k) {
-    return ((unsigned long long)__float_as_uint(t) << 32) | k;
+// A hit's key: its distance, its candidate's number (at most 2^24) and, in the
+// low five bits, how far beyond the distance other hits matter: up to `near`,
+// the near distance of the boxes above it, rounded up to 2^bits - 1 units in
+// the last place (0: not beyond; at most 2^29, a factor of 2^64).
+SLIM_D unsigned long long hit_key(float t, float near, uint32_t k) {
+    const uint32_t beyond = __float_as_uint(maxr(t, near)) - __float_as_uint(t);
+    return ((unsigned long long)__float_as_uint(t) << 32) | (k << 5) | min(32u - (uint32_t)__clz((int)beyond), 29u);
 }
 SLIM_D float key_distance(unsigned long long key) { return __uint_as_float((uint32_t)(key >> 32)); }
+SLIM_D float key_reach(unsigned long long key) {
+    uint32_t beyond;                // 2^bits - 1; the width wraps to its low five bits
+    asm("bmsk.wrap.b32 %0, 0, %1;" : "=r"(beyond) : "r"((uint32_t)key));
+    return __uint_as_float((uint32_t)(key >> 32) + beyond);
+}
 // No hit yet: distance +inf.
-constexpr unsigned long long kNoHitKey = (0x7F800000ull << 32) | 0xFFFFFFFFull;
+constexpr unsigned long long kNoHitKey = (0x7F800000ull << 32) | 0xFFFFFFE0ull;
 
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F0, QueueArgs A) {
@@ -789,6 +800,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
         hit.distance = INFINITY;
         int best_geo = -1;
         uint32_t best_k = 0, k = 0;
+        float best_near = 0.0f;         // near distance of the boxes above the best implicit hit
         bool full = false;
         // A visible mesh instance of a leaf with near and far distances ln, lf:
         // a candidate, or a single-leaf mesh's triangles here.
@@ -821,6 +833,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
                     mh.uv_coverage = __ldg(&S.tri_cold[4 * (size_t)(m.tri_offset + mh.id) + 3].w);
                     best_geo = (int)gi;
                     best_k = k;
+                    best_near = maxr(ln, rn);
                     hit = mh;
                     hit.NdotRd = -(dot(hit.normal, local.d));
                 }
@@ -833,10 +846,11 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
             p[0] = make_float4(local.o.x, local.o.y, local.o.z, clip);
             p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(slot));
             p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
-            p[3] = make_float4(__uint_as_float(gi), __uint_as_float(g.mesh), __uint_as_float(k), 0.0f);
+            p[3] = make_float4(__uint_as_float(gi), __uint_as_float(g.mesh), __uint_as_float(k),
+                               copysignf(maxr(ln, rn), -1.0f));
         };
-        // one scene leaf: [first, first + count) geometries, far distance lf
-        auto leaf = [&](uint32_t first, uint32_t count, float lf) {
+        // one scene leaf: [first, first + count) geometries, near and far distances ln, lf
+        auto leaf = [&](uint32_t first, uint32_t count, float ln, float lf) {
             Hit aux;
             aux.distance = minr(lf + kEps, hit.distance);
             Ray local;
@@ -845,11 +859,12 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
                 Geo g = load_geo(S, gi);
                 if (!(g.flags & SLIM_GEOMETRY_IS_VISIBLE)) continue;
                 if (g.type == SLIM_GEOMETRY_MESH) {
-                    instance(gi, g, 0.0f, lf, nullptr);
+                    instance(gi, g, ln, lf, nullptr);
                 } else if (hit_geometry_local<COUNT>(S, g, r, local, aux, false, nullptr, err, w) &&
                            aux.distance < hit.distance) {
                     best_geo = (int)gi;
                     best_k = k;
+                    best_near = ln;
                     hit = aux;
                     hit.NdotRd = -(dot(hit.normal, local.d));
                 }
@@ -858,8 +873,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
         // Small scenes: every leaf's box, then the implicit primitives of the
         // hit ones, then their mesh instances, the best implicit hit already
         // known.  Candidates are numbered in that order from 1; an implicit hit
-        // has 0, and a candidate at exactly the ray's best distance that is not
-        // its holder sends the ray to the whole walk (k_extend_resolve).
+        // has 0.
         const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
         if (!COUNT && list.x && finite_ray(r)) {
             const uint32_t leaves = leaves_hit(S, list.x, r, INFINITY, list.y | list.z);
@@ -881,6 +895,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
                 }
             }
             best_k = 0;
+            best_near = seen.near;
             full |= seen.unsure;
         } else {
         float ln, rn, lf, rf;
@@ -889,7 +904,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
         bump<COUNT>(w.scene_nodes);
         if (hit_node(r, a, b, ln, lf) && ln < hit.distance) {
             if (node_leaf_count(b)) {
-                leaf(0, S.geometry_count, lf);
+                leaf(0, S.geometry_count, ln, lf);
             } else {
                 uint32_t left = node_first(b), top = 0;
                 for (;;) {
@@ -902,11 +917,11 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
                     uint32_t lchild = node_first(lb), rchild = node_first(xb);
                     bool go_left = hl, go_right = hr;
                     if (hl && node_leaf_count(lb)) {
-                        leaf(lchild, node_leaf_count(lb), lf);
+                        leaf(lchild, node_leaf_count(lb), ln, lf);
                         go_left = false;
                     }
                     if (hr && node_leaf_count(xb)) {
-                        leaf(rchild, node_leaf_count(xb), rf);
+                        leaf(rchild, node_leaf_count(xb), rn, rf);
                         go_right = false;
                     }
                     if (go_left) {
@@ -934,7 +949,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
             A.masks[slot] = 0ull;
             overflow[atomicAdd(A.pair_count + 2, 1u)] = slot;
         } else {
-            A.masks[slot] = best_geo >= 0 ? hit_key(hit.distance, best_k) : kNoHitKey;
+            A.masks[slot] = best_geo >= 0 ? hit_key(hit.distance, best_near, best_k) : kNoHitKey;
             store_hit(A.hits, A.hit_stride, slot, best_geo, hit);
         }
     }
@@ -975,7 +990,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
     bool busy = false;
     uint32_t idx = 0, slot = 0, top = 0, bottom = 0, tri_offset = 0, tri = 0, k = 0;
     uint32_t next = kNone, waiting = kNone;
-    float lc = 0.0f, lc_near = 0.0f, reach = 0.0f, bu = 0.0f, bv = 0.0f;
+    float lc = 0.0f, lc_near = 0.0f, box_near = 0.0f, reach = 0.0f, bu = 0.0f, bv = 0.0f;
     bool found = false, behind = false, unsure = false;
     bool piece = false, shared = false;     // part of another lane's walk; a walk that gave parts away
     Ray r;
@@ -997,7 +1012,8 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
     };
     // the ray's other candidates and, of a shared walk, its other parts cull by
     // the published distance; two with the same leave the ray undecided
-    auto publish = [&]() { unsure |= key_distance(atomicMin(A.masks + slot, hit_key(lc, k))) == lc; };
+    auto key = [&]() { return hit_key(lc, maxr(lc_near, box_near), k); };
+    auto publish = [&]() { unsure |= key_distance(atomicMin(A.masks + slot, key())) == lc; };
     // candidate i from its root, or from a node of its walk
     auto start = [&](uint32_t i, uint32_t from) {
         const float4 *p = A.pairs + 4 * (size_t)i;
@@ -1011,10 +1027,11 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
         idx = i;
         reset(r, xyz(p0), xyz(p1));
         wr = wide_setup(r, p2.z);
-        lc = p0.w;
+        lc = lc_near = p0.w;
+        box_near = fabsf(p3.w);
         slot = __float_as_uint(p1.w);
         k = __float_as_uint(p3.z);
-        reach = fminf(lc, key_distance(A.masks[slot])) * kReachSlack;
+        reach = fminf(lc, key_reach(A.masks[slot])) * kReachSlack;
         next = __float_as_uint(p2.x);
         waiting = kNone;
         tri_offset = __float_as_uint(p2.y);
@@ -1093,7 +1110,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
             float ln, lf;
             waiting = kNone;
             if (wide_leaf_box(r, wr, na, nb, ln, lf)) {
-                const float gb = key_distance(A.masks[slot]);
+                const float gb = key_reach(A.masks[slot]);
                 const float before = lc;
                 const uint32_t count = node_leaf_count(nb), first = node_first(nb);
                 for (uint32_t i = 0; i < count; i++) {
@@ -1121,7 +1138,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                     found = true;
                 }
                 if (SHARE && shared && lc < before) publish();
-                reach = fminf(lc, gb) * kReachSlack;
+                reach = fminf(lc_near, gb) * kReachSlack;
             }
             advance();
         }
@@ -1133,14 +1150,14 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                 // publishes and waits for no answer (waiting: 225 -> 284 us for the first round's launch)
                 if (found && !unsure) {
                     p[2] = result;
-                    p[3].w = 1.0f;
-                    atomicMin(A.masks + slot, hit_key(lc, k));
+                    p[3].w = maxr(lc_near, box_near);
+                    atomicMin(A.masks + slot, key());
                 }
             } else if (found && !unsure) {
                 const unsigned long long held = __ldcg(A.masks + slot);
-                const bool best = held == hit_key(lc, k);
+                const bool best = held == key();
                 // not the nearest, but where the order of the visits decides
-                unsure = !best && lc == key_distance(held);
+                unsure = !best && held && lc <= key_reach(held);
                 uint32_t record = idx;
                 if (best && piece) {
                     // a part's hit gets a record of its own behind the candidates
@@ -1152,7 +1169,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                     const float4 p1 = p[1], p3 = p[3];
                     if (piece) o[1] = p1;
                     o[2] = result;
-                    o[3] = make_float4(p3.x, p3.y, p3.z, 1.0f);
+                    o[3] = make_float4(p3.x, p3.y, p3.z, maxr(lc_near, box_near));
                 }
             }
             // two hits so close together that the order of the visits decides
@@ -1186,16 +1203,25 @@ __global__ void __launch_bounds__(256) k_extend_resolve(DevScene S0, DevFrame F0
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
         const float4 *p = A.pairs + 4 * (size_t)idx;
         const float4 p3 = p[3];
-        if (p3.w == 0.0f) continue;
+        if (signbit(p3.w)) continue;
         const float4 p1 = p[1], p2 = p[2];
         const uint32_t slot = __float_as_uint(p1.w);
         const unsigned long long best = A.masks[slot];
-        if (best != hit_key(p2.x, __float_as_uint(p3.z))) {
-            // two candidates at the same distance: the order of the visits decides
-            if ((uint32_t)(best >> 32) == __float_as_uint(p2.x) && best && atomicExch(A.masks + slot, 0ull))
+        const bool winner = best == hit_key(p2.x, p3.w, __float_as_uint(p3.z));
+        // the hit that is not the nearest: another candidate's here, or the best
+        // implicit one
+        float other = p2.x;
+        if (winner) {
+            other = INFINITY;
+            if ((best & 31u) && __float_as_int(A.hits[2 * (size_t)A.hit_stride + slot].x) >= 0) other = A.hits[slot].w;
+        }
+        if (best && other <= key_reach(best) && other < INFINITY) {
+            // so close to the nearest that the order of the visits decides
+            if (atomicExch(A.masks + slot, 0ull))
                 reinterpret_cast<uint32_t *>(A.shadow_rays)[atomicAdd(A.pair_count + 2, 1u)] = slot;
             continue;
         }
+        if (!winner) continue;
         uint32_t pid = 0;
         if (BATCH) pid = __float_as_uint(A.rays_in[2 * (size_t)slot + 1].w);
         const DevScene &S = scene_of<BATCH>(S0, A, pid);

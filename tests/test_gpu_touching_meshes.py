@@ -22,7 +22,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 REPEATS = 4
-IN_A_BOX = ("in a box",)
+IN_A_BOX = ("in a box", "in a box, grouped")
 
 
 def asset(builder, shift=0.0, raised=0):
@@ -66,6 +66,9 @@ def touching_scene(kind, turned, far, side, distance):
     elif kind in IN_A_BOX:          # on its floor, seen from inside; the mesh's leaf comes first or second
         put(L.GEOMETRY_BOX, 0, (2.0, 1.0, 2.0), 0, (0.5 * side, 1.0, 0.0))
         put(L.GEOMETRY_MESH, 1)
+        if kind == "in a box, grouped":     # the mesh's leaf is further down the BVH than the box's
+            for x in (-0.3, 0.2, 0.4):
+                put(L.GEOMETRY_SPHERE, 2, (0.05, 0.05, 0.05), 0, (x, 0.2, -0.9))
     elif kind == "mesh on quad":
         put(L.GEOMETRY_QUAD, 0, (1.3, 1.0, 1.1))
         put(L.GEOMETRY_MESH, 1, (1.0, 1.0, 1.0), 0)
