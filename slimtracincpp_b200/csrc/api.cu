@@ -632,6 +632,7 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
     if (rc) return rc;
     c.scene.meshes = c.d_meshes.ptr;
     c.scene.mesh_count = n;
+    c.scene.binary_walks = 0;
     if (!n) {
         c.scene.mesh_nodes = nullptr;
         c.scene.tri_hot = c.scene.tri_cold = nullptr;
@@ -672,6 +673,7 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
                              cudaMemcpyHostToDevice), "upload triangle attributes");
         dm.wide_root = build_wide_bvh(m.bvh.nodes, m.bvh.node_count, &hot[0].x, kStackCapacity, wide, wide_leaves,
                                       dm.wide_extent);
+        c.scene.binary_walks |= dm.wide_root == kNoWideBVH && !m.bvh.nodes[0].leaf_count;
     }
     SLIM_CUDA(cudaMemcpy(c.d_meshes.ptr, metas.data(), metas.size() * sizeof(DevMesh), cudaMemcpyHostToDevice), "upload meshes");
     if ((rc = c.d_wide_nodes.reserve(wide.size() ? wide.size() : 1, "alloc wide nodes"))) return rc;

@@ -95,6 +95,7 @@ struct DevScene {
     uint32_t flags;                // SLIM_SCENE_HAD_EMISSIVE_QUADS
     uint32_t scene_node_count;
     const LeafList *leaves;
+    uint32_t binary_walks;         // a mesh has no wide form: the mesh walks take the binary BVHs
 };
 
 // Per-frame parameters of a render launch.

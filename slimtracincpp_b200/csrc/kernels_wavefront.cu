@@ -116,7 +116,7 @@ struct QueueArgs {
     uint32_t *shadow_count;
     unsigned long long *masks;    // per slot: bit i = light i occluded
     float4 *pairs;                // shadow ray x mesh instance candidates, 3 float4 each:
-                                  // (local origin, aux distance) (local direction, tag) (wide root, triangles, plane bound, 0)
+                                  // (local origin, aux distance) (local direction, tag) (walk_record)
     uint32_t *pair_count;
     uint32_t *pair_cursor;
     uint32_t pair_capacity;
@@ -312,6 +312,14 @@ __global__ void __launch_bounds__(256) k_shadow_gen(DevScene S0, DevFrame F0, Qu
 //                 pair as soon as its own finishes, so warps stay full
 //                 although walk lengths differ by orders of magnitude.
 
+// Where the walk of a mesh with root node bytes `root` starts, for its record.
+SLIM_D float4 walk_record(const DevScene &S, const DevMesh &m, float4 root) {
+    if (S.binary_walks)
+        return make_float4(__uint_as_float(m.node_offset + node_first(root)), __uint_as_float(m.tri_offset),
+                           __uint_as_float(m.node_offset), 0.0f);
+    return make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
+}
+
 SLIM_D bool local_box_test(const DevScene &S, const Geo &g, const Ray &local) {
     float mn[3], mx[3], n, f;
     if (g.type == SLIM_GEOMETRY_MESH) {
@@ -362,15 +370,15 @@ SLIM_D bool shadow_leaf(const DevScene &S, const QueueArgs &A, uint32_t tag, uin
                     if (hit_triangles<COUNT>(S.tri_hot, m.tri_offset, m.tri_count, lf2, local, h, true, w)) return true;
                     break;
                 }
-                const bool wide = m.wide_root != kNoWideBVH;
-                uint32_t slot = warp_append(A.pair_count, wide);
-                if (wide && slot < A.pair_capacity) {
+                const bool queued = S.binary_walks || m.wide_root != kNoWideBVH;
+                uint32_t slot = warp_append(A.pair_count, queued);
+                if (queued && slot < A.pair_capacity) {
                     float4 *p = A.pairs + 3 * (size_t)slot;
                     p[0] = make_float4(local.o.x, local.o.y, local.o.z, aux);
                     p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(tag));
-                    p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
+                    p[2] = walk_record(S, m, rb);
                 } else if (mesh_trace<COUNT>(S, m, local, h, true, mesh_stack, err, w)) {
-                    return true;   // no wide walk, or the pair queue is full: trace the instance here
+                    return true;   // the pair queue is full: trace the instance here
                 }
             } break;
             default: break;
@@ -561,7 +569,7 @@ struct Steal {
     bool gave;
     uint32_t subtree, near;     // stack entry handed over (valid for a taker)
 };
-template <typename Entry>
+template <bool NEAR, typename Entry>
 SLIM_D Steal steal_round(uint32_t idle_mask, uint32_t donor_mask, const Entry *stack, uint32_t &bottom, uint32_t &top) {
     const uint32_t below = (1u << lane_id()) - 1u;
     const uint32_t pairs = min((uint32_t)__popc(idle_mask), (uint32_t)__popc(donor_mask));
@@ -579,26 +587,51 @@ SLIM_D Steal steal_round(uint32_t idle_mask, uint32_t donor_mask, const Entry *s
     for (uint32_t j = 0; taker && j < my_idle_rank; j++) m &= m - 1u;
     const int src = taker ? __ffs((int)m) - 1 : (int)lane_id();
     st.subtree = __shfl_sync(0xFFFFFFFFu, give.x, src);
-    st.near = sizeof(Entry) == sizeof(uint2) ? __shfl_sync(0xFFFFFFFFu, give.y, src) : 0u;
+    st.near = NEAR ? __shfl_sync(0xFFFFFFFFu, give.y, src) : 0u;
     st.from = taker ? src : -1;
     return st;
 }
 
+// Scenes with a mesh that has no wide form (boxes that do not nest, or a walk
+// that could have too many nodes waiting) walk every mesh's binary BVH in the
+// same loops, one pair of children and their exact boxes per step (WIDE false).
+// The 1080p frame of the 81,920- and 130,050-triangle meshes with one box of
+// each outside its parent's: 1.32 ms, against 1.15 with the wide form and 3.24
+// when such rays were traced whole.  A walk's references are then nodes: of an
+// inner one the first child, of a leaf kWideLeaf | itself.
+SLIM_D uint32_t binary_child(uint32_t node_offset, uint32_t i, float4 b) {
+    return node_leaf_count(b) ? kWideLeaf | i : node_offset + node_first(b);
+}
+// Children i and i + 1 of an inner node against the ray, as wide_hits but exactly.
+SLIM_D uint32_t binary_hits(const DevScene &S, uint32_t node_offset, uint32_t i, const Ray &r, float tmax,
+                            uint32_t child[2], float t0[2], float t1[2]) {
+    uint32_t hits = 0;
+#pragma unroll
+    for (uint32_t s = 0; s < 2; s++) {
+        float4 a, b;
+        load_node(S.mesh_nodes, i + s, a, b);
+        child[s] = binary_child(node_offset, i + s, b);
+        if (hit_node(r, a, b, t0[s], t1[s]) && t0[s] < tmax) hits |= 1u << s;
+    }
+    return hits;
+}
+
 // The hot record of triangle i of a leaf whose first triangle is `first`:
-// the first two lie in the leaf's own line.
+// the first two lie in a wide leaf's own line.
+template <bool WIDE>
 SLIM_D const float4 *leaf_triangle(const DevScene &S, const float4 *leaf, uint32_t first, uint32_t i) {
-    return i < 2 ? leaf + 2 + 3 * i : S.tri_hot + 3 * (size_t)(first + i);
+    return WIDE && i < 2 ? leaf + 2 + 3 * i : S.tri_hot + 3 * (size_t)(first + i);
 }
 
 // MeshTracer::hitTriangles (mesh_tracer.h:23-49) over a wide leaf, any hit
 // closer than `closest`.
-template <bool COUNT>
+template <bool COUNT, bool WIDE>
 SLIM_D bool any_triangle(const DevScene &S, const float4 *leaf, uint32_t tri_offset, float4 node, float closest,
                          const Ray &r, Work &w) {
     const uint32_t count = node_leaf_count(node), first = tri_offset + node_first(node);
     for (uint32_t i = 0; i < count; i++) {
         bump<COUNT>(w.triangles);
-        const float4 *t4 = leaf_triangle(S, leaf, first, i);
+        const float4 *t4 = leaf_triangle<WIDE>(S, leaf, first, i);
         const float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
         const float3 p = xyz(a), n = f3(a.w, b.x, b.y);
         float t; float3 pos; bool behind;
@@ -611,14 +644,14 @@ SLIM_D bool any_triangle(const DevScene &S, const float4 *leaf, uint32_t tri_off
     return false;
 }
 
-template <bool COUNT>
+template <bool COUNT, bool WIDE>
 __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_mesh(DevScene S, DevFrame F, QueueArgs A) {
     chain_wait();
     Feed feed(min(*A.pair_count, A.pair_capacity));
     uint32_t stack[kStackCapacity];
     Work w = {};
     bool busy = false, hit = false;
-    uint32_t idx = 0, tag = 0, top = 0, bottom = 0, tri_offset = 0;
+    uint32_t idx = 0, tag = 0, top = 0, bottom = 0, tri_offset = 0, node_offset = 0;
     uint32_t next = kNone;          // node or leaf the walk goes to
     uint32_t waiting = kNone;       // a leaf to be tested
     float aux = 0.0f;
@@ -641,7 +674,8 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
         if ((A.masks[tag >> 6] >> (tag & 63u)) & 1ull) return;   // already known occluded
         idx = i;
         reset(r, xyz(p0), xyz(p1));
-        wr = wide_setup(r, p2.z);
+        if constexpr (WIDE) wr = wide_setup(r, p2.z);
+        else node_offset = __float_as_uint(p2.z);
         aux = p0.w;
         tri_offset = __float_as_uint(p2.y);
         next = from == kNone ? __float_as_uint(p2.x) : from;
@@ -669,7 +703,7 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
                 const uint32_t i = feed.take(A.pair_cursor, idle);
                 if (i < feed.n) start(i, kNone);
             } else if (donors) {
-                const Steal st = steal_round(idle, donors, stack, bottom, top);
+                const Steal st = steal_round<false>(idle, donors, stack, bottom, top);
                 const uint32_t from_idx = __shfl_sync(0xFFFFFFFFu, idx, st.from >= 0 ? st.from : (int)lane_id());
                 if (st.from >= 0) start(from_idx, st.subtree);
             } else if (feed.drained && idle == 0xFFFFFFFFu) {
@@ -682,15 +716,16 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
                 // One node of the any-hit walk: the hit child that reaches
                 // furthest is next (a shadow ray's occluder is rarely the
                 // surface it starts on), the others go on the stack.
-                uint4 child;
-                float t0[4], t1[4];
-                const uint32_t hits = wide_hits(S.wide_nodes, next, r, wr, aux, child, t0, t1);
-                bump<COUNT>(w.mesh_nodes, 4);
+                constexpr int kChildren = WIDE ? 4 : 2;
+                uint32_t c[kChildren], hits;
+                float t0[kChildren], t1[kChildren];
+                if constexpr (WIDE) hits = wide_hits(S.wide_nodes, next, r, wr, aux, c, t0, t1);
+                else hits = binary_hits(S, node_offset, next, r, aux, c, t0, t1);
+                bump<COUNT>(w.mesh_nodes, kChildren);
                 next = kNone;
                 float reach = -1.0f;
-                const uint32_t c[4] = {child.x, child.y, child.z, child.w};
 #pragma unroll
-                for (int s = 0; s < 4; s++)
+                for (int s = 0; s < kChildren; s++)
                     if (hits >> s & 1u) {
                         const bool further = t1[s] > reach;
                         const uint32_t other = further ? next : c[s];
@@ -702,12 +737,14 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
             }
         }
         if (leaf_round(waiting != kNone, busy && !(next & kWideLeaf)) && waiting != kNone) {
-            const float4 *leaf = S.wide_leaves + 8 * (size_t)(waiting & ~kWideLeaf);
+            const float4 *leaf = WIDE ? S.wide_leaves + 8 * (size_t)(waiting & ~kWideLeaf)
+                                      : S.mesh_nodes + 2 * (size_t)(waiting & ~kWideLeaf);
             float4 a, b;
             load_node(leaf, 0, a, b);
             float ln, lf;
             waiting = kNone;
-            if (wide_leaf_box(r, wr, a, b, ln, lf) && ln < aux && any_triangle<COUNT>(S, leaf, tri_offset, b, minr(lf, aux), r, w)) {
+            if ((WIDE ? wide_leaf_box(r, wr, a, b, ln, lf) : hit_node(r, a, b, ln, lf)) && ln < aux &&
+                any_triangle<COUNT, WIDE>(S, leaf, tri_offset, b, minr(lf, aux), r, w)) {
                 atomicOr(A.masks + (tag >> 6), 1ull << (tag & 63u));
                 hit = true;
                 next = kNone;
@@ -756,11 +793,11 @@ __global__ void __launch_bounds__(kMeshBlock, SLIM_SHADOW_MESH_BLOCKS) k_shadow_
 // but in the held hit's reach, leaves the ray undecided, as do parts with hits
 // at the same distance or with a hit that is not beyond its box's near distance.
 // Candidate records (4 float4): (local origin, clip) (local direction, slot)
-// (wide root, triangle offset, plane bound, 0) (geometry, mesh, k, -near), near
-// being the near distance of the boxes above the mesh; a walk that ends with a
-// hit overwrites the third with (t, u, v, triangle | behind << 31) and the last
-// word with the hit's own near distance, sign clear.  The ray keys live in the
-// shadow-mask array, which is free until the shadow stage.
+// (walk_record) (geometry, mesh, k, -near), near being the near distance of the
+// boxes above the mesh; a walk that ends with a hit overwrites the third with
+// (t, u, v, triangle | behind << 31) and the last word with the hit's own near
+// distance, sign clear.  The ray keys live in the shadow-mask array, which is
+// free until the shadow stage.
 
 // A hit's key: its distance, its candidate's number (at most 2^24) and, in the
 // low five bits, how far beyond the distance other hits matter: up to `near`,
@@ -839,13 +876,13 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
                 }
                 return;
             }
-            const bool wide = m.wide_root != kNoWideBVH;
-            uint32_t q = warp_append(A.pair_count, wide);
-            if (!wide || q >= cap) { full = true; return; }
+            const bool queued = S.binary_walks || m.wide_root != kNoWideBVH;
+            uint32_t q = warp_append(A.pair_count, queued);
+            if (!queued || q >= cap) { full = true; return; }
             float4 *p = A.pairs + 4 * (size_t)q;
             p[0] = make_float4(local.o.x, local.o.y, local.o.z, clip);
             p[1] = make_float4(local.d.x, local.d.y, local.d.z, __uint_as_float(slot));
-            p[2] = make_float4(__uint_as_float(m.wide_root), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
+            p[2] = walk_record(S, m, rb);
             p[3] = make_float4(__uint_as_float(gi), __uint_as_float(g.mesh), __uint_as_float(k),
                                copysignf(maxr(ln, rn), -1.0f));
         };
@@ -983,23 +1020,34 @@ __global__ void __launch_bounds__(256) k_extend_overflow(DevScene S0, DevFrame F
     flush_stage<COUNT>(A.counters, w);
 }
 
-template <bool COUNT, bool SHARE>
+template <bool COUNT, bool SHARE, bool WIDE>
 SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint32_t cap) {
     uint2 stack[kStackCapacity];    // (node or leaf, its near distance)
     Work w = {};
     bool busy = false;
-    uint32_t idx = 0, slot = 0, top = 0, bottom = 0, tri_offset = 0, tri = 0, k = 0;
+    uint32_t idx = 0, slot = 0, top = 0, bottom = 0, tri_offset = 0, node_offset = 0, tri = 0, k = 0;
     uint32_t next = kNone, waiting = kNone;
     float lc = 0.0f, lc_near = 0.0f, box_near = 0.0f, reach = 0.0f, bu = 0.0f, bv = 0.0f;
     bool found = false, behind = false, unsure = false;
     bool piece = false, shared = false;     // part of another lane's walk; a walk that gave parts away
+    // Binary boxes need not nest: near distances of `next` and `waiting` are
+    // then the largest of the boxes on the way there, and `margin` is the slab
+    // test's rounding, which wide boxes have in them.
+    float next_near = 0.0f, waiting_near = 0.0f, margin = 0.0f;
     Ray r;
     WideRay wr;
+    auto slack = [&](float t) {
+        if constexpr (WIDE) return t * kReachSlack;
+        else return t * kReachSlack + margin;
+    };
     // the nearest waiting entry that can still hold a closer hit
     auto pop = [&]() -> uint32_t {
         while (top > bottom) {
             const uint2 e = stack[--top];
-            if (__uint_as_float(e.y) <= reach) return e.x;
+            if (__uint_as_float(e.y) <= reach) {
+                if (!WIDE) next_near = __uint_as_float(e.y);
+                return e.x;
+            }
         }
         return kNone;
     };
@@ -1007,6 +1055,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
         if (next == kNone) next = pop();
         if (next != kNone && (next & kWideLeaf) && waiting == kNone) {
             waiting = next;
+            if (!WIDE) waiting_near = next_near;
             next = pop();
         }
     };
@@ -1015,23 +1064,30 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
     auto key = [&]() { return hit_key(lc, maxr(lc_near, box_near), k); };
     auto publish = [&]() { unsure |= key_distance(atomicMin(A.masks + slot, key())) == lc; };
     // candidate i from its root, or from a node of its walk
-    auto start = [&](uint32_t i, uint32_t from) {
+    auto start = [&](uint32_t i, uint32_t from, float near) {
         const float4 *p = A.pairs + 4 * (size_t)i;
         const float4 p0 = p[0], p1 = p[1], p3 = p[3];
         float4 p2 = p[2];
         piece = shared = SHARE && from != kNone;
         if (piece) {        // the walk's own result may have taken the place of its mesh
             const DevMesh &m = S.meshes[__float_as_uint(p3.y)];
-            p2 = make_float4(__uint_as_float(from), __uint_as_float(m.tri_offset), m.wide_extent, 0.0f);
+            p2 = make_float4(__uint_as_float(from), __uint_as_float(m.tri_offset),
+                             WIDE ? m.wide_extent : __uint_as_float(m.node_offset), 0.0f);
         }
         idx = i;
         reset(r, xyz(p0), xyz(p1));
-        wr = wide_setup(r, p2.z);
+        if constexpr (WIDE) {
+            wr = wide_setup(r, p2.z);
+        } else {
+            node_offset = __float_as_uint(p2.z);
+            margin = slab_margin(r);
+            next_near = near;
+        }
         lc = lc_near = p0.w;
         box_near = fabsf(p3.w);
         slot = __float_as_uint(p1.w);
         k = __float_as_uint(p3.z);
-        reach = fminf(lc, key_reach(A.masks[slot])) * kReachSlack;
+        reach = slack(fminf(lc, key_reach(A.masks[slot])));
         next = __float_as_uint(p2.x);
         waiting = kNone;
         tri_offset = __float_as_uint(p2.y);
@@ -1051,7 +1107,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                 base = __shfl_sync(active, base, leader);
                 const uint32_t i = base + (uint32_t)__popc(active & ((1u << lane_id()) - 1u));
                 if (i >= feed.n) break;
-                start(i, kNone);
+                start(i, kNone, 0.0f);
             }
         } else {
             const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
@@ -1059,9 +1115,9 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                 const uint32_t donors = feed.donors(busy && top > bottom);
                 if (feed.fetch(idle, donors)) {
                     const uint32_t i = feed.take(A.pair_cursor, idle);
-                    if (i < feed.n) start(i, kNone);
+                    if (i < feed.n) start(i, kNone, 0.0f);
                 } else if (donors) {
-                    const Steal st = steal_round(idle, donors, stack, bottom, top);
+                    const Steal st = steal_round<!WIDE>(idle, donors, stack, bottom, top);
                     if (st.gave) {
                         // a hit at or before its own box's near distance is sure
                         // only against hits of the same lane
@@ -1070,7 +1126,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                         shared = true;
                     }
                     const uint32_t from_idx = __shfl_sync(0xFFFFFFFFu, idx, st.from >= 0 ? st.from : (int)lane_id());
-                    if (st.from >= 0) start(from_idx, st.subtree);
+                    if (st.from >= 0) start(from_idx, st.subtree, __uint_as_float(st.near));
                 } else if (feed.drained && idle == 0xFFFFFFFFu) {
                     break;
                 }
@@ -1081,16 +1137,21 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
         if (SHARE) __syncwarp();
 #pragma unroll
         for (uint32_t sub = 0; sub < kStepsPerTurn; sub++) if (busy && !(next & kWideLeaf)) {
-            uint4 child;
-            float t0[4], t1[4];
-            const uint32_t hits = wide_hits(S.wide_nodes, next, r, wr, reach, child, t0, t1);
-            bump<COUNT>(w.mesh_nodes, 4);
+            constexpr int kChildren = WIDE ? 4 : 2;
+            uint32_t c[kChildren], hits;
+            float t0[kChildren], t1[kChildren];
+            if constexpr (WIDE) {
+                hits = wide_hits(S.wide_nodes, next, r, wr, reach, c, t0, t1);
+            } else {
+                hits = binary_hits(S, node_offset, next, r, reach, c, t0, t1);
+                for (float &t : t0) t = maxr(t, next_near);
+            }
+            bump<COUNT>(w.mesh_nodes, kChildren);
             // the nearest hit child is next, the others go on the stack
             float near = INFINITY;
             next = kNone;
-            const uint32_t c[4] = {child.x, child.y, child.z, child.w};
 #pragma unroll
-            for (int s = 0; s < 4; s++)
+            for (int s = 0; s < kChildren; s++)
                 if (hits >> s & 1u) {
                     const bool nearer = t0[s] < near;
                     const uint32_t other = nearer ? next : c[s];
@@ -1099,23 +1160,26 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                     near = nearer ? t0[s] : near;
                     if (other != kNone) stack[top++] = make_uint2(other, __float_as_uint(far));
                 }
+            if (!WIDE) next_near = near;
             advance();
         }
         if (SHARE) __syncwarp();
         if (leaf_round(waiting != kNone, busy && !(next & kWideLeaf)) && waiting != kNone) {
             // MeshTracer::hitTriangles (mesh_tracer.h:23-49) with the leaf's far clip
-            const float4 *leaf = S.wide_leaves + 8 * (size_t)(waiting & ~kWideLeaf);
+            const float4 *leaf = WIDE ? S.wide_leaves + 8 * (size_t)(waiting & ~kWideLeaf)
+                                      : S.mesh_nodes + 2 * (size_t)(waiting & ~kWideLeaf);
             float4 na, nb;
             load_node(leaf, 0, na, nb);
             float ln, lf;
             waiting = kNone;
-            if (wide_leaf_box(r, wr, na, nb, ln, lf)) {
+            if (WIDE ? wide_leaf_box(r, wr, na, nb, ln, lf) : hit_node(r, na, nb, ln, lf)) {
+                if (!WIDE) ln = maxr(ln, waiting_near);
                 const float gb = key_reach(A.masks[slot]);
                 const float before = lc;
                 const uint32_t count = node_leaf_count(nb), first = node_first(nb);
                 for (uint32_t i = 0; i < count; i++) {
                     bump<COUNT>(w.triangles);
-                    const float4 *t4 = leaf_triangle(S, leaf, tri_offset + first, i);
+                    const float4 *t4 = leaf_triangle<WIDE>(S, leaf, tri_offset + first, i);
                     float4 a = __ldg(t4), b = __ldg(t4 + 1), c = __ldg(t4 + 2);
                     float3 pp = xyz(a), nn = f3(a.w, b.x, b.y);
                     float tt; float3 pos; bool bh;
@@ -1138,7 +1202,7 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
                     found = true;
                 }
                 if (SHARE && shared && lc < before) publish();
-                reach = fminf(lc_near, gb) * kReachSlack;
+                reach = slack(fminf(lc_near, gb));
             }
             advance();
         }
@@ -1183,13 +1247,13 @@ SLIM_D void extend_walks(const DevScene &S, const QueueArgs &A, Feed &feed, uint
     flush_stage<COUNT>(A.counters, w);
 }
 
-template <bool COUNT>
+template <bool COUNT, bool WIDE>
 __global__ void __launch_bounds__(kMeshBlock, SLIM_EXTEND_MESH_BLOCKS) k_extend_mesh(DevScene S, DevFrame F, QueueArgs A) {
     chain_wait();
     const uint32_t cap = A.pair_capacity * 3u / 4u;
     Feed feed(min(*A.pair_count, cap));
-    if (feed.sparse()) extend_walks<COUNT, true>(S, A, feed, cap);
-    else extend_walks<COUNT, false>(S, A, feed, cap);
+    if (feed.sparse()) extend_walks<COUNT, true, WIDE>(S, A, feed, cap);
+    else extend_walks<COUNT, false, WIDE>(S, A, feed, cap);
 }
 
 // The candidate holding its ray's minimum (distance, k) writes the hit
@@ -1756,8 +1820,8 @@ cudaError_t trace_round(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         A.pair_cursor = counts + 2;
         L.launch(!primary, k_extend_scene<COUNT, BATCH>,
                  L.grid((const void *)k_extend_scene<COUNT, BATCH>, L.bound), L.block, S, F, A);
-        L.launch(true, k_extend_mesh<COUNT>,
-                 L.mesh_grid((const void *)k_extend_mesh<COUNT>, B.pair_capacity), kMeshBlock, S, F, A);
+        const auto extend_mesh = S.binary_walks ? k_extend_mesh<COUNT, false> : k_extend_mesh<COUNT, true>;
+        L.launch(true, extend_mesh, L.mesh_grid((const void *)extend_mesh, B.pair_capacity), kMeshBlock, S, F, A);
         L.launch(true, k_extend_resolve<COUNT, BATCH>,
                  L.grid((const void *)k_extend_resolve<COUNT, BATCH>, B.pair_capacity), L.block, S, F, A);
         L.launch(true, k_extend_overflow<COUNT, BATCH>,
@@ -1808,8 +1872,8 @@ cudaError_t trace_round(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         if (!L.split_extend) continue;
         A.counters = L.stage(STAGE_SHADOW_MESH);
         if (timer) timer->begin(STAGE_SHADOW_MESH, stream);
-        L.launch(true, k_shadow_mesh<COUNT>,
-                 L.mesh_grid((const void *)k_shadow_mesh<COUNT>, B.pair_capacity), kMeshBlock, S, F, A);
+        const auto shadow_mesh = S.binary_walks ? k_shadow_mesh<COUNT, false> : k_shadow_mesh<COUNT, true>;
+        L.launch(true, shadow_mesh, L.mesh_grid((const void *)shadow_mesh, B.pair_capacity), kMeshBlock, S, F, A);
         if (timer) timer->end(STAGE_SHADOW_MESH, stream);
     }
     if (L.pixel_wait && (r = cudaStreamWaitEvent(stream, L.pixel_wait, 0)) != cudaSuccess) return r;

@@ -43,11 +43,14 @@ SLIM_D WideRay wide_setup(Ray &r, float extent) {     // r.rcp becomes the walk'
 
 // Four children of wide node i against the ray: bit s of the result is set
 // when box s is hit before tmax, between t0[s] and t1[s].
-SLIM_D uint32_t wide_hits(const uint4 *nodes, uint32_t i, const Ray &r, const WideRay &w, float tmax, uint4 &child,
-                          float t0[4], float t1[4]) {
+SLIM_D uint32_t wide_hits(const uint4 *nodes, uint32_t i, const Ray &r, const WideRay &w, float tmax,
+                          uint32_t child[4], float t0[4], float t1[4]) {
     const uint4 *n = nodes + 5 * (size_t)i;
-    const uint4 a = __ldg(n), c = __ldg(n + 2), d = __ldg(n + 3), e = __ldg(n + 4);
-    child = __ldg(n + 1);
+    const uint4 a = __ldg(n), b = __ldg(n + 1), c = __ldg(n + 2), d = __ldg(n + 3), e = __ldg(n + 4);
+    child[0] = b.x;
+    child[1] = b.y;
+    child[2] = b.z;
+    child[3] = b.w;
     const float3 org = f3(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
     const float3 near = mul_add(org, r.rcp, w.near), far = mul_add(org, r.rcp, w.far);
     const uint32_t nx[2] = {r.nx ? d.z : c.x, r.nx ? d.w : c.y}, fx[2] = {r.nx ? c.x : d.z, r.nx ? c.y : d.w};
