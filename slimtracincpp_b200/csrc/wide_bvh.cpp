@@ -71,10 +71,19 @@ float wide_offset(const uint32_t words[2], int s) {
     return from_bits(s & 1 ? words[s >> 1] : words[s >> 1] << 16);
 }
 
+uint32_t most_wide_nodes(const SlimBVHNode *nodes, uint32_t node_count) {
+    uint32_t inner = 0;
+    for (uint32_t i = 0; i < node_count; i++) inner += !nodes[i].leaf_count;
+    return (uint32_t)((2ull * inner + 1) / 3);
+}
+
 uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const float *hot, uint32_t stack,
                         std::vector<WideNode> &out, std::vector<WideLeaf> &leaves, float &extent) {
     if (!node_count || nodes[0].leaf_count || !boxes_nest(nodes, node_count)) return kNoWideBVH;
     const size_t root = out.size(), first_leaf = leaves.size();
+    const size_t most = most_wide_nodes(nodes, node_count);
+    size_t leaf_nodes = 0;
+    for (uint32_t i = 0; i < node_count; i++) leaf_nodes += nodes[i].leaf_count != 0;
     std::vector<uint32_t> source{0};       // binary node of every wide node from `root` on
     std::vector<uint32_t> waiting{0};      // nodes a walk may have waiting when it enters it
     source.reserve(node_count / 2);
@@ -137,7 +146,8 @@ uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const flo
             }
         }
         out.push_back(n);
-        if (waiting[w] + count - 1 > stack || leaves.size() >= kWideLeaf || root + source.size() >= kWideLeaf) {
+        if (waiting[w] + count - 1 > stack || leaves.size() >= kWideLeaf || root + source.size() >= kWideLeaf ||
+            source.size() > most || leaves.size() - first_leaf > leaf_nodes) {      // no tree
             out.resize(root);
             leaves.resize(first_leaf);
             return kNoWideBVH;

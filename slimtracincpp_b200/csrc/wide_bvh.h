@@ -44,11 +44,18 @@ float wide_offset(const uint32_t words[2], int s);
 // inner node) to `out` and `leaves` and returns the index of its root.
 // `hot` holds 12 floats per triangle.  Returns kNoWideBVH, appending nothing,
 // when a node's box does not hold its children's boxes or a plane is not
-// finite (or beyond 1e18), which the argument above needs, or when a walk
-// could have more than `stack` nodes waiting.  `extent`: no plane of the
-// form, rounded or not, is further from the mesh's origin.
+// finite (or beyond 1e18), which the argument above needs, when a walk could
+// have more than `stack` nodes waiting, or when nodes share children, so that
+// the form would hold many copies of them.  `extent`: no plane of the form,
+// rounded or not, is further from the mesh's origin.
 uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const float *hot, uint32_t stack,
                         std::vector<WideNode> &out, std::vector<WideLeaf> &leaves, float &extent);
+
+// Most nodes the wide form of a binary BVH can have.  A wide node with four
+// children takes the place of three inner nodes, one with fewer has leaves only;
+// with F of the former and P of the latter, P <= 3 F + 1 and there are at least
+// 3 F + P inner nodes.
+uint32_t most_wide_nodes(const SlimBVHNode *nodes, uint32_t node_count);
 
 // Every box finite (within 1e18) and inside its parent's: a slab test that
 // passes for a node then passes for everything above it.
