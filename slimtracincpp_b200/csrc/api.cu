@@ -640,8 +640,20 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
         c.scene.wide_leaves = nullptr;
         return SLIM_OK;
     }
+    // The wide form's arrays are as large as BVHs with as many inner nodes and
+    // leaves can need, so that like the others they stay in place when meshes
+    // of the same sizes are uploaded again (a captured frame holds their
+    // addresses).
+    size_t most_wide = 0, most_leaves = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        const SlimBVH &b = s->meshes[i].bvh;
+        most_wide += most_wide_nodes(b.nodes, b.node_count);
+        for (uint32_t k = 0; k < b.node_count; k++) most_leaves += b.nodes[k].leaf_count != 0;
+    }
     std::vector<WideNode> wide;
     std::vector<WideLeaf> wide_leaves;
+    wide.reserve(most_wide);
+    wide_leaves.reserve(most_leaves);
     rc = c.d_mesh_nodes.reserve(2 * total_nodes, "alloc mesh nodes");
     if (rc) return rc;
     rc = c.d_tri_hot.reserve(3 * total_tris, "alloc triangles");
@@ -676,8 +688,8 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
         c.scene.binary_walks |= dm.wide_root == kNoWideBVH && !m.bvh.nodes[0].leaf_count;
     }
     SLIM_CUDA(cudaMemcpy(c.d_meshes.ptr, metas.data(), metas.size() * sizeof(DevMesh), cudaMemcpyHostToDevice), "upload meshes");
-    if ((rc = c.d_wide_nodes.reserve(wide.size() ? wide.size() : 1, "alloc wide nodes"))) return rc;
-    if ((rc = c.d_wide_leaves.reserve(wide_leaves.size() ? wide_leaves.size() : 1, "alloc wide leaves"))) return rc;
+    if ((rc = c.d_wide_nodes.reserve(most_wide ? most_wide : 1, "alloc wide nodes"))) return rc;
+    if ((rc = c.d_wide_leaves.reserve(most_leaves ? most_leaves : 1, "alloc wide leaves"))) return rc;
     if (!wide.empty()) {
         SLIM_CUDA(cudaMemcpy(c.d_wide_nodes.ptr, wide.data(), wide.size() * sizeof(WideNode), cudaMemcpyHostToDevice),
                   "upload wide nodes");

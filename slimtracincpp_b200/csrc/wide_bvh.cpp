@@ -88,8 +88,6 @@ uint32_t build_wide_bvh(const SlimBVHNode *nodes, uint32_t node_count, const flo
     std::vector<uint32_t> waiting{0};      // nodes a walk may have waiting when it enters it
     source.reserve(node_count / 2);
     waiting.reserve(node_count / 2);
-    out.reserve(root + node_count / 3);
-    leaves.reserve(first_leaf + node_count / 2 + 1);
     for (size_t w = 0; w < source.size(); w++) {
         // open the largest inner child until four are reached
         uint32_t child[4], count = 0;
