@@ -224,7 +224,10 @@ enum { SLIM_CACHE_OFF = 0, SLIM_CACHE_ON = 1, SLIM_CACHE_TRUNCATE = 2, SLIM_CACH
 /* Work counters of the last frame (rays traced and memory records touched).
  * The shadow_* fields are the parts of the node, triangle and geometry
  * tests spent in any-hit (shadow-ray) traversals; only the fused engine,
- * which walks every ray in the reference's order, splits them out. */
+ * which walks every ray in the reference's order, splits them out.  A counting
+ * frame walks the scene BVH, which other frames of small scenes do not (they
+ * test its leaves one by one), and counts four boxes per node of a mesh's
+ * four-wide BVH, empty slots included. */
 typedef struct {
     uint64_t primary_rays, shadow_rays, bounce_rays;
     uint64_t scene_node_tests, mesh_node_tests, triangle_tests;

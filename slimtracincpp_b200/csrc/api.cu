@@ -601,7 +601,7 @@ int upload_meshes(Context &c, const SlimSceneData *s) {
         if (rc) return rc;
         if (m.triangle_count >= (1u << kLeafCountShift))
             return set_error(SLIM_ERR_LIMIT, "mesh has 2^26 triangles or more");
-        for (uint32_t k = 1; k < m.bvh.node_count; k++)   // a root leaf is tested without being packed
+        for (uint32_t k = 1; k < m.bvh.node_count; k++)   // a root leaf may hold any number
             if (m.bvh.nodes[k].leaf_count >= (1u << (32 - kLeafCountShift)))
                 return set_error(SLIM_ERR_LIMIT, "mesh BVH leaf below the root holds 64 triangles or more");
         uint32_t d = bvh_depth(m.bvh.nodes, m.bvh.node_count);

@@ -27,7 +27,8 @@ namespace slim {
 constexpr int kStackCapacity = 64;        // per-ray traversal stack entries (scene and mesh)
 // Meshes hold fewer than 2^26 triangles and leaves below the root fewer than
 // 64 (checked on upload; the reference's builder makes leaves of at most
-// two).
+// two).  No record packs the two into one word any more; meshes beyond stay
+// refused as before.
 constexpr uint32_t kLeafCountShift = 26;
 constexpr int kMaxLights = 64;            // lights a shadow mask can track
 constexpr uint32_t kErrStack = 1u;        // device error bits

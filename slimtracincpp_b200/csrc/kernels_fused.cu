@@ -39,7 +39,7 @@ SLIM_D void render_sample(const DevScene &S, const DevFrame &F, int x, int y, ui
         float3 color = f3(0, 0, 0);
         float depth = INFINITY;
         Surface s;
-        int g = scene_trace<COUNT>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+        int g = scene_trace<COUNT>(S, F.width * F.rows, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
         if (g >= 0) {
             Geo geo = load_geo(S, (uint32_t)g);
             Mat m = load_mat(S, geo.material);
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(128) k_trace_primary(DevScene S, SlimCameraRay
     Ray ray;
     reset(ray, f3(P.camera_position.x, P.camera_position.y, P.camera_position.z), normalized(primary_direction(P, x, y)));
     Hit hit;
-    int g = scene_trace<false>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+    int g = scene_trace<false>(S, width * height, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
     geometry_ids[i] = g;
     bool mesh = false;
     if (g >= 0) mesh = load_geo(S, (uint32_t)g).type == SLIM_GEOMETRY_MESH;
@@ -216,7 +216,7 @@ __global__ void k_pick(DevScene S, SlimCameraRayProjection P, int x, int y, Slim
     Ray ray;
     reset(ray, f3(P.camera_position.x, P.camera_position.y, P.camera_position.z), normalized(primary_direction(P, x, y)));
     Hit hit;
-    int g = scene_trace<false>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+    int g = scene_trace<false>(S, 1, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
     float max_distance = hit.distance;
     int light = -1;
     for (uint32_t i = 0; i < S.light_count; i++) {

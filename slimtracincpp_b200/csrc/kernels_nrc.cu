@@ -630,8 +630,8 @@ cudaError_t launch_train_step(const float4 *features, const float4 *targets, uin
     count_launch();
     AdamArgs a = adam;
     a.parts = (uint32_t)g;
-    k_nrc_adam<<<(kParams + kAdamParams - 1) / kAdamParams, kAdamParams * kAdamParts, 0, stream>>>(params, adam_m, adam_v, partials, loss_partials, grad, loss,
-                                                          weight_image, a, samples, count, offset);
+    k_nrc_adam<<<(kParams + kAdamParams - 1) / kAdamParams, kAdamParams * kAdamParts, 0, stream>>>(
+        params, adam_m, adam_v, partials, loss_partials, grad, loss, weight_image, a, samples, count, offset);
     count_launch();
     return cudaGetLastError();
 }

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) k_extend(DevScene S0, DevFrame F0, QueueA
         Ray ray;
         reset(ray, o, d);
         Hit hit;
-        int g = scene_trace<COUNT>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+        int g = scene_trace<COUNT>(S, n, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
         store_hit(A.hits, A.hit_stride, slot, g, hit);
     }
     if (err) atomicOr(F0.error_flags, err);
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
         bool occluded = false;
         float ln, rn, lf, rf;
         float4 ra, rb;
-        const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
+        const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S, n);
         if (!COUNT && list.x && finite_ray(ray)) {
             for (uint32_t leaves = leaves_hit(S, list.x, ray, Ld, list.w); leaves && !occluded; leaves &= leaves - 1u) {
                 load_leaf(S, __ffs((int)leaves) - 1, ra, rb);
@@ -911,7 +911,7 @@ __global__ void __launch_bounds__(256, 2) k_extend_scene(DevScene S0, DevFrame F
         // hit ones, then their mesh instances, the best implicit hit already
         // known.  Candidates are numbered in that order from 1; an implicit hit
         // has 0.
-        const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
+        const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S, n);
         if (!COUNT && list.x && finite_ray(r)) {
             const uint32_t leaves = leaves_hit(S, list.x, r, INFINITY, list.y | list.z);
             Nearest seen;
@@ -1013,7 +1013,7 @@ __global__ void __launch_bounds__(256) k_extend_overflow(DevScene S0, DevFrame F
         Ray ray;
         reset(ray, o, d);
         Hit hit;
-        int g = scene_trace<COUNT>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+        int g = scene_trace<COUNT>(S, n, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
         store_hit(A.hits, A.hit_stride, slot, g, hit);
     }
     if (err) atomicOr(F0.error_flags, err);
@@ -1341,7 +1341,7 @@ __global__ void __launch_bounds__(128) k_finish_paths(DevScene S0, DevFrame F0, 
             Hit hit;
             float3 current = f3(0, 0, 0), next_throughput = f3(0, 0, 0);
             bool bounce = false;
-            int g = scene_trace<COUNT>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+            int g = scene_trace<COUNT>(S, n, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
             float hit_distance = INFINITY;
             if (g >= 0) {
                 hit_distance = hit.distance;
@@ -1362,7 +1362,7 @@ __global__ void __launch_bounds__(128) k_finish_paths(DevScene S0, DevFrame F0, 
                             sr.d = s.L;
                             Hit sh;
                             bump<COUNT>(w.shadow);
-                            if (scene_trace<COUNT>(S, sr, sh, true, s.Ld, stack, mesh_stack, err, w) >= 0) continue;
+                            if (scene_trace<COUNT>(S, n, sr, sh, true, s.Ld, stack, mesh_stack, err, w) >= 0) continue;
                         }
                         add_light(s, m, l, current);
                     }
@@ -1732,8 +1732,11 @@ struct RoundLaunch {
     // us; signalled from the start of each kernel instead of from its end, the
     // waiting blocks keep the other band off the SMs: 2.050 and 1.124 ms).
     // The first launch of a frame is not chained, so that the scene it reads
-    // through the read-only path is complete; neither are launches that follow
-    // an event or are captured into a graph.
+    // through the read-only path is complete; neither are launches that wait for
+    // an event of another stream or are captured into a graph.  (An event
+    // recorded between two launches of the stream changes nothing: it marks the
+    // end of the first, and the second writes nothing before that.)  A launch's
+    // error is the last error, which each round checks.
     bool chain = false;
     template <typename... P, typename... X>
     void launch(bool chained, void (*kernel)(P...), uint32_t grid, int threads, const X &...args) const {

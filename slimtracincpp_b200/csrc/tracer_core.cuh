@@ -53,7 +53,6 @@ SLIM_D float3 scale_add(float3 a, float f, float3 b) { return f3(fmaf(a.x, f, b.
 SLIM_D float3 mul_add(float3 a, float3 m, float3 b) { return f3(fmaf(a.x, m.x, b.x), fmaf(a.y, m.y, b.y), fmaf(a.z, m.z, b.z)); }
 SLIM_D float3 one_minus(float3 a) { return f3(1.0f - a.x, 1.0f - a.y, 1.0f - a.z); }
 SLIM_D float3 reflected(float3 d, float3 n) { return scale_add(n, -2.0f * dot(d, n), d); }
-SLIM_D float3 ld3(const float *p) { return f3(__ldg(p), __ldg(p + 1), __ldg(p + 2)); }
 SLIM_D float3 xyz(float4 v) { return f3(v.x, v.y, v.z); }
 
 // quat * vec3 (math/quat.h:37-43)
@@ -541,9 +540,26 @@ SLIM_D int hit_geometries(const DevScene &S, uint32_t first, uint32_t count, flo
     return hit_geo;
 }
 
-// The first words of a scene's leaf list: how many, which hold visible implicit
-// primitives, visible mesh instances, anything that casts shadows.
-SLIM_D uint4 listed_leaves(const DevScene &S) { return __ldg(reinterpret_cast<const uint4 *>(S.leaves)); }
+// The first words of a scene's leaf list: how many (0: walk the tree), which
+// hold visible implicit primitives, visible mesh instances, anything that casts
+// shadows.  A launch of few rays waits for its longest walks, which the list
+// shortens at every length; one of many is bound by instructions, and a box per
+// leaf and ray becomes more of them than the tree's steps.  Where depends on
+// the scene: objects scattered over the view, list against tree, in us,
+//   leaves                        8       12        16        24        32
+//   fused, 1280x720, depth 1    91/92    98/96   108/103   132/120   151/130
+//   fused, 427x241, depth 4     46/50    47/48    57/62     66/71     88/94
+//   stages, 1920x1080, depth 4 254/255  269/265  292/284   344/318   390/337
+//   stages, 427x241, depth 4    79/83    83/92    99/111   133/146   153/184
+// but the textured scene's 13 leaves close together 394/420 at 1920x1080 and the
+// mesh scene's 9 1122/1200.
+constexpr uint32_t kManyRays = 1u << 18;
+constexpr uint32_t kListedForMany = 16;
+SLIM_D uint4 listed_leaves(const DevScene &S, uint32_t rays) {
+    uint4 list = __ldg(reinterpret_cast<const uint4 *>(S.leaves));
+    if (rays > kManyRays && list.x > kListedForMany) list.x = 0;
+    return list;
+}
 SLIM_D void load_leaf(const DevScene &S, uint32_t j, float4 &a, float4 &b) {
     load_node(reinterpret_cast<const float4 *>(S.leaves->leaf), j, a, b);
 }
@@ -631,13 +647,14 @@ SLIM_D int closest_of_leaves(const DevScene &S, uint32_t leaves, const Ray &r, H
 
 // SceneTracer::trace (scene_tracer.h:26-98): offsets the origin by
 // TRACE_OFFSET along the direction, then walks the scene BVH near child
-// first (both children tested per step, the far one pushed).
+// first (both children tested per step, the far one pushed).  `rays`: how many
+// the launch traces (listed_leaves).
 template <bool COUNT>
-SLIM_D int scene_trace(const DevScene &S, Ray &r, Hit &hit, bool any_hit, float max_distance,
+SLIM_D int scene_trace(const DevScene &S, uint32_t rays, Ray &r, Hit &hit, bool any_hit, float max_distance,
                        uint32_t *stack, uint32_t *mesh_stack, uint32_t &err, Work &w) {
     reset(r, scale_add(r.d, kTraceOffset, r.o), r.d);
     hit.distance = max_distance;
-    const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S);
+    const uint4 list = COUNT ? make_uint4(0, 0, 0, 0) : listed_leaves(S, rays);
     if (!COUNT && list.x && (any_hit || !S.mesh_count) && finite_ray(r)) {
         uint32_t leaves = leaves_hit(S, list.x, r, max_distance, any_hit ? list.w : list.y);
         if (any_hit) {
@@ -1232,7 +1249,8 @@ SLIM_D bool path_segment(const DevScene &S, const DevFrame &F, PathState &p, uin
     Hit hit;
     Surface s;
     float3 current = f3(0, 0, 0), next_throughput = f3(0, 0, 0);
-    int g = scene_trace<COUNT>(S, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
+    const uint32_t rays = F.width * F.rows;
+    int g = scene_trace<COUNT>(S, rays, ray, hit, false, INFINITY, stack, mesh_stack, err, w);
     if (g >= 0) {
         Geo geo = load_geo(S, (uint32_t)g);
         Mat m = load_mat(S, geo.material);
@@ -1252,7 +1270,7 @@ SLIM_D bool path_segment(const DevScene &S, const DevFrame &F, PathState &p, uin
                     Hit sh;
                     bump<COUNT>(w.shadow);
                     const uint32_t sn = w.scene_nodes, mn = w.mesh_nodes, tr = w.triangles, ge = w.geometries;
-                    const bool occluded = scene_trace<COUNT>(S, sr, sh, true, s.Ld, stack, mesh_stack, err, w) >= 0;
+                    const bool occluded = scene_trace<COUNT>(S, rays, sr, sh, true, s.Ld, stack, mesh_stack, err, w) >= 0;
                     bump<COUNT>(w.any_scene_nodes, w.scene_nodes - sn);
                     bump<COUNT>(w.any_mesh_nodes, w.mesh_nodes - mn);
                     bump<COUNT>(w.any_triangles, w.triangles - tr);
