@@ -319,12 +319,20 @@ __global__ void __launch_bounds__(128 * kGroups, 2) k_nrc_infer(const float4 *__
 }
 
 // ---- training -----------------------------------------------------------------
-// Samples of a step: `n` from `offset` on, clipped to the device count when
-// one is given (the frame's training set size is only known on the device).
-SLIM_N uint32_t step_samples(uint32_t n, const uint32_t *count, uint32_t offset) {
-    if (!count) return n;
-    uint32_t c = *count;
-    return c > offset ? (c - offset < n ? c - offset : n) : 0u;
+// Samples of a step: `n` of them, or -- the frame's training set, whose size is
+// only known on the device -- part `offset / n` of the `count` in as many parts
+// of up to `n` as that takes.  The parts are dealt out in turn: a set lies in
+// the order in which the frame's blocks appended its queries, so parts one after
+// the other would each cover a region of the picture, the last, shortest one
+// with as much weight as the first.
+struct StepSamples {
+    uint32_t n, first, stride;
+    SLIM_N uint32_t at(uint32_t i) const { return first + i * stride; }
+};
+SLIM_N StepSamples step_samples(uint32_t n, const uint32_t *count, uint32_t offset) {
+    if (!count) return {n, 0, 1};
+    const uint32_t total = *count, parts = (total + n - 1) / n, part = offset / n;
+    return {part < parts ? (total - part + parts - 1) / parts : 0u, part, parts};
 }
 
 __global__ void __launch_bounds__(128, 1) k_nrc_train(const float4 *__restrict__ features,
@@ -344,11 +352,10 @@ __global__ void __launch_bounds__(128, 1) k_nrc_train(const float4 *__restrict__
     __shared__ int abort_s;
     __shared__ float loss_s[4];
     const uint32_t t = threadIdx.x, warp = t >> 5;
-    const uint32_t n = step_samples(n_max, count, offset);
+    const StepSamples samples = step_samples(n_max, count, offset);
+    const uint32_t n = samples.n;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     if (n && blockIdx.x == 0 && t == 0) atomicAdd(step, 1u);
-    features += 4 * (size_t)offset;
-    targets += offset;
     for (uint32_t i = t; i < kImgBytes / 16; i += blockDim.x)
         ((uint4 *)W)[i] = ((const uint4 *)weight_image)[i];
     if (t == 0) { mbar_init(&bar, 1); abort_s = 0; }
@@ -372,8 +379,9 @@ __global__ void __launch_bounds__(128, 1) k_nrc_train(const float4 *__restrict__
     for (uint32_t tile = blockIdx.x; tile < tiles && !aborted; tile += gridDim.x) {
         const uint32_t i = tile * kTile + t;
         const bool valid = i < n;
-        encode_row(features + 4 * (size_t)i, valid, X, t);
-        float4 y = valid ? targets[i] : make_float4(0, 0, 0, 0);
+        const size_t row = samples.at(i);
+        encode_row(features + 4 * row, valid, X, t);
+        float4 y = valid ? targets[row] : make_float4(0, 0, 0, 0);
         sync_for_mma();
         // forward
         for (int l = 0; l < 5 && !aborted; l++) {
@@ -532,7 +540,7 @@ __global__ void __launch_bounds__(kAdamParams * kAdamParts) k_nrc_adam(
     __shared__ float quarter[kAdamParts][kAdamParams];
     const uint32_t k = threadIdx.x % kAdamParams, q = threadIdx.x / kAdamParams;
     const uint32_t p = blockIdx.x * kAdamParams + k;
-    const uint32_t n = step_samples(n_max, count, offset);
+    const uint32_t n = step_samples(n_max, count, offset).n;
     if (!n) return;                                  // empty step: no update
     const uint32_t rows = (a.parts + kAdamParts - 1) / kAdamParts, first = q * rows;
     const uint32_t end = min(first + rows, a.parts);

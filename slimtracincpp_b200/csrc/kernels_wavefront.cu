@@ -1977,6 +1977,17 @@ cudaError_t trace_training(const RoundLaunch &L, QueueArgs &A, const CacheArgs &
     return cudaGetLastError();
 }
 
+// The Adam steps over a frame's training set, as many as a full set takes; a
+// step past the parts of the set as it is changes nothing.
+cudaError_t train_steps(const CacheFrame *cache, cudaStream_t stream) {
+    const uint32_t n = cache->batch < cache->train_capacity ? cache->batch : cache->train_capacity;
+    for (uint32_t off = 0; off < cache->train_capacity; off += n) {
+        const cudaError_t e = cache->trainer->step(cache->t_features, cache->t_targets, n, cache->counts + 1, off, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // After the queries of a frame (or wave) are gathered: the training paths
 // traced on (to max_depth, or a few bounces into the cache's own answers),
 // the Adam steps, the network's answers, and the waiting paths resolved.
@@ -2028,12 +2039,7 @@ cudaError_t cache_phase(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
         TA.samples = TB.capacity;
         if ((e = trace_training<false, false>(TL, TA, CA, 0, cache, max_depth, cache->train_weights)) != cudaSuccess)
             return e;
-        for (uint32_t off = 0; off < cache->train_capacity; off += cache->batch) {
-            uint32_t n = cache->train_capacity - off < cache->batch ? cache->train_capacity - off : cache->batch;
-            if ((e = cache->trainer->step(cache->t_features, cache->t_targets, n, cache->counts + 1, off, ts)) !=
-                cudaSuccess)
-                return e;
-        }
+        if ((e = train_steps(cache, ts)) != cudaSuccess) return e;
         if ((e = cudaEventRecord(cache->trained, ts)) != cudaSuccess) return e;
     } else if (mode == SLIM_CACHE_EXACT || train) {
         if (timer) timer->begin(STAGE_CACHE, stream);
@@ -2057,12 +2063,7 @@ cudaError_t cache_phase(const RoundLaunch &L, QueueArgs &A, const CacheArgs &CA,
     }
     if (train && !(cache->train_stream && cache->train_queues && !BATCH)) {
         if (timer) timer->begin(STAGE_CACHE_TRAIN, stream);
-        for (uint32_t off = 0; off < cache->train_capacity; off += cache->batch) {
-            uint32_t n = cache->train_capacity - off < cache->batch ? cache->train_capacity - off : cache->batch;
-            if ((e = cache->trainer->step(cache->t_features, cache->t_targets, n, cache->counts + 1, off, stream)) !=
-                cudaSuccess)
-                return e;
-        }
+        if ((e = train_steps(cache, stream)) != cudaSuccess) return e;
         if (timer) timer->end(STAGE_CACHE_TRAIN, stream);
     }
     if (mode == SLIM_CACHE_ON) {

@@ -54,11 +54,11 @@ int train_grid(uint32_t samples, bool beside_a_frame);
 cudaError_t launch_infer(const float4 *features, const uint32_t *count, uint32_t n, uint32_t capacity,
                          float4 *radiance, const uint8_t *weight_image, uint32_t *error_flags, cudaStream_t stream);
 
-// One optimisation step over the (features, targets) pairs [offset, offset +
-// samples), clipped to *count when `count` (a device counter) is given:
-// gradients of the mean log-radiance L2 loss into grad (f32, kParams), Adam update
-// of params / m / v, refreshed bf16 image, loss into *loss.  A step with no
-// samples changes nothing.
+// One optimisation step over the first `samples` (features, targets) pairs, or
+// over part offset / samples of the *count pairs when `count` (a device counter)
+// is given (StepSamples): gradients of the mean log-radiance L2 loss into grad
+// (f32, kParams), Adam update of params / m / v, refreshed bf16 image, loss into
+// *loss.  A step with no samples changes nothing.
 cudaError_t launch_train_step(const float4 *features, const float4 *targets, uint32_t samples, const uint32_t *count,
                               uint32_t offset, float *params, float *adam_m, float *adam_v, uint8_t *weight_image,
                               float *partials, float *loss_partials, float *grad, float *loss, const AdamArgs &adam,
