@@ -618,14 +618,14 @@ template <bool COUNT>
 SLIM_D int closest_of_leaves(const DevScene &S, uint32_t leaves, const Ray &r, Hit &hit, Nearest &seen, uint32_t &err,
                              Work &w) {
     int best = -1;
-    const float margin = slab_margin(r);
+    float limit = INFINITY;         // leaves beginning beyond hold no hit that matters
     while (leaves) {
         float4 a, b;
         float ln, lf;
         load_leaf(S, __ffs((int)leaves) - 1, a, b);
         leaves &= leaves - 1u;
         hit_box_finite(r, a, b, ln, lf);
-        if (ln > seen.reach(hit.distance) * kReachSlack + margin) continue;
+        if (ln > limit) continue;
         const uint32_t first = node_first(b), count = node_leaf_count(b);
         Hit aux;
         for (uint32_t i = 0; i < count; i++) {
@@ -639,6 +639,7 @@ SLIM_D int closest_of_leaves(const DevScene &S, uint32_t leaves, const Ray &r, H
                 best = (int)gi;
                 hit = aux;
                 hit.NdotRd = -(dot(hit.normal, local.d));
+                limit = seen.reach(hit.distance) * kReachSlack + slab_margin(r);
             }
         }
     }
