@@ -232,16 +232,15 @@ def reference_order_stage_bytes(w):
             "shadow_mesh": 32 * w["shadow_mesh_node_tests"] + 64 * w["shadow_triangle_tests"]}
 
 
-# Cache-level utilisation of the persistent mesh walks, from one
-#   ncu --set full --clock-control none -k regex:<kernel> -s 2 -c 1
-# launch each (config 2, 1920x1080, whole-frame passes; profiles/ holds the table): L1TEX and L2 (lts) throughput as
-# a share of their hardware peaks.  The walks read nodes and triangles mostly from L1 (72-77 % hit rate) and wait on
-# the latency of those dependent loads: L1 runs at half to three quarters of its peak, L2 at a tenth.
+# Cache-level utilisation of the persistent mesh walks' first-round launches, from an ncu capture of one whole frame
+# (config 2, 1920x1080; profiles/ holds the command and the table): L1TEX and L2 (lts) throughput as a share of their
+# hardware peaks.  The walks read nodes and triangles mostly from L1 (71-72 % hit rate) and issue in 55-68 % of the
+# cycles at 14-18 lanes of 32: L1 runs at 37-55 % of its peak, L2 at 11-14 %.
 MEMORY_LEVELS = {
-    "config2": {"k_extend_mesh": {"l1tex_throughput_pct": 50.9, "lts_throughput_pct": 10.4, "l1tex_hit_pct": 77.0,
-                                  "warps_active_pct": 35.1, "threads_per_instruction": 16.3},
-                "k_shadow_mesh": {"l1tex_throughput_pct": 72.8, "lts_throughput_pct": 15.1, "l1tex_hit_pct": 72.3,
-                                  "warps_active_pct": 52.5, "threads_per_instruction": 18.6}},
+    "config2": {"k_extend_mesh": {"l1tex_throughput_pct": 37.3, "lts_throughput_pct": 10.6, "l1tex_hit_pct": 72.1,
+                                  "warps_active_pct": 34.1, "threads_per_instruction": 14.3},
+                "k_shadow_mesh": {"l1tex_throughput_pct": 55.2, "lts_throughput_pct": 13.8, "l1tex_hit_pct": 71.3,
+                                  "warps_active_pct": 46.9, "threads_per_instruction": 18.2}},
 }
 
 
@@ -250,8 +249,8 @@ MEMORY_LEVELS = {
 # on the bench's own command (profiles/ holds the per-kernel table).  ncu flushes caches before every kernel, so
 # these are cold-cache bytes.  A stage launch is all kernels of one round: extend = scene + mesh + resolve + overflow.
 TRAFFIC_BYTES_PER_LAUNCH = {
-    ("config2", "extend"): 180.0e6,       # rounds 1 and 2: 259 MB and 101 MB
-    ("config2", "shadow_mesh"): 61.6e6,   # 93.0 MB and 30.2 MB
+    ("config2", "extend"): 155.5e6,       # rounds 1 and 2: 207 MB and 104 MB
+    ("config2", "shadow_mesh"): 62.6e6,   # 96.3 MB and 28.9 MB
 }
 PIXEL_STAGES = ("shade", "tail", "fused")   # stages that write the framebuffer
 CACHE_WARMUP_FRAMES = 32   # radiance-cache frames trained before the timed ones
@@ -979,10 +978,11 @@ def main():
                     "share_of_frame": d["total_ms"] / prof_ms,
                     "timing": "CUDA events around every launch of the stage, whole-frame passes (row_bands=1)",
                     "memory_levels": {"kernels": MEMORY_LEVELS.get(args.config),
-                                      "source": "ncu --set full, one launch per kernel, cold caches",
-                                      "note": "the scene's nodes and triangles (34 MB) stay in the 126 MB L2 and "
-                                              "mostly hit L1: the walks are bound by dependent-load latency, "
-                                              "with L1TEX at 51-73 % and L2 at 10-15 % of peak throughput"}}
+                                      "source": "ncu, the first round's launches of a whole frame, cold caches",
+                                      "note": "the scene's nodes and triangles (53 MB, 19 MB of them the four-wide "
+                                              "BVHs) stay in the 126 MB L2 and mostly hit L1: the walks are bound by "
+                                              "instructions at 14-18 busy lanes of 32 and by dependent loads, with "
+                                              "L1TEX at 37-55 % and L2 at 11-14 % of peak throughput"}}
     frame_bytes = algorithmic_bytes(work)
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,

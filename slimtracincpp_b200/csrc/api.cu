@@ -908,11 +908,12 @@ int wait_for_refit(Context &c, cudaStream_t stream) {
 
 // Frames of fewer samples than this in scenes without meshes run the fused
 // kernel under SLIM_ENGINE_AUTO even when their paths bounce.  Measured on
-// one B200, render only, the fused kernel against the wavefront engine:
-// config 1's implicit scene (paths end at the first hit) 0.031 / 0.050 ms at
-// 320x180, 0.036 / 0.069 at 640x360, 0.105 / 0.129 at 1280x720, 0.209 /
-// 0.258 at 1920x1080; config 3's glass, mirror and texture scene at depth 8
-// 0.075 / 0.163, 0.109 / 0.192, 0.274 / 0.260, 0.506 / 0.449 ms.
+// one B200, whole calls by events, the fused kernel against the wavefront
+// engine: the implicit scene (paths end at the first hit) 44 / 53 us at
+// 320x180, 51 / 72 at 640x360, 111 / 135 at 1280x720, 202 / 244 at 1920x1080;
+// the glass, mirror and texture scene at depth 8 71 / 121, 96 / 148, 215 / 243
+// and 423 / 394 us.  (The line stood between 640x360 and 1280x720 before the
+// leaf lists came; it would now lie between the last two sizes.)
 constexpr uint64_t kAutoFusedSamples = 1u << 19;
 
 // The engine a frame runs on: the option, or under SLIM_ENGINE_AUTO the

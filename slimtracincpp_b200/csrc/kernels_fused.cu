@@ -78,15 +78,14 @@ SLIM_D void render_sample(const DevScene &S, const DevFrame &F, int x, int y, ui
 // Blocks per SM the fused kernel is compiled for (register caps with
 // spills that mostly hit L1), one build for frames whose paths end at their
 // first hit (no reflective or refractive material, or max depth 1) and one
-// for the rest.  Measured on one B200, frames without refit, blocks per SM
-// for short / long paths:
-//   4 / 4 (128 registers):  config 1 640x360 0.035 ms, 1920x1080 0.201;
-//                           config 3 (glass, depth 8) 320x180 0.075, 640x360 0.107
-//   5 / 4:                  config 1 0.039, 0.215
-//   6 / 4:                  config 1 0.041, 0.217
-//   4 / 3 (170 registers):  config 3 0.071, 0.107
-//   4 / 5:                  config 3 0.082, 0.123
-// (uncapped, 220 registers and two blocks: config 1 0.045 ms).
+// for the rest.  Measured on one B200, whole calls by events, in us:
+//   blocks              3      4      5
+//   implicit, 640x360   52     51     54      (short paths)
+//   implicit, 1080p    213    202    208
+//   blocks              2      3      4
+//   glass, 320x180      69     71     76      (long paths, depth 8)
+//   glass, 640x360     108     96     98
+//   glass, 1280x720    245    215    218
 #ifndef SLIM_FUSED_SHORT_BLOCKS
 #define SLIM_FUSED_SHORT_BLOCKS 4
 #endif

@@ -229,8 +229,8 @@ SLIM_N void sync_for_mma() {
 // 64 TMEM columns: 24 KB of shared memory and an eighth of the columns a tile.
 // 1,036,801 samples: 196 us with two tiles per SM, 149 us with six, 102 us with
 // packed conversions (pack2) besides, 97 us with packed ReLUs (relu2).  It now
-// issues in 56 % of the cycles (73.7 M warp instructions before relu2), more
-// than half of that for the 36 sincospif of a sample.
+// issues in 61 % of the cycles (60.0 M warp instructions, 73.7 M before relu2),
+// more than half of that for the 36 sincospif of a sample.
 constexpr uint32_t kGroups = 3;
 SLIM_N void group_sync(uint32_t group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory"); }
 SLIM_N void group_sync_for_mma(uint32_t group) {

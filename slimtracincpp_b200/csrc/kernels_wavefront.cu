@@ -387,10 +387,9 @@ SLIM_D bool shadow_leaf(const DevScene &S, const QueueArgs &A, uint32_t tag, uin
     return false;
 }
 
-// Capped at 64 registers (4 blocks per SM instead of 3): latency-bound, the
-// extra warps pay for the few spills (config 2: shadow 0.157 -> 0.149 ms;
-// re-measured on the final build, 3 blocks at 78 registers without spills:
-// 0.155 against 0.148 ms).
+// Capped at 64 registers (4 blocks per SM): latency-bound, the extra warps pay
+// for the few spills.  With 3 blocks the mesh frame at 1080p takes 1.149 ms and
+// the textured one 393 us, with 4 1.147 and 394, with 5 1.153 and 400.
 #ifndef SLIM_SHADOW_SCENE_BLOCKS
 #define SLIM_SHADOW_SCENE_BLOCKS 4
 #endif
@@ -480,8 +479,9 @@ __global__ void __launch_bounds__(256, SLIM_SHADOW_SCENE_BLOCKS) k_shadow_scene(
 //   eight-wide, 8-bit planes, 80 B, 9.0 nodes         238 M, L1 50 %, 321 us
 //   four-wide, 32-bit planes, 112 B read, 13 nodes    169 M, L1 83 %, 328 us
 //   four-wide, 16-bit planes, 80 B, 11.7 nodes        201 M, L1 67 %, 292 us (this)
-// (the last also goes to the child that reaches furthest first).  The frame:
-// 1.455 -> 1.283 ms; with 8 bounces 2.865 -> 2.550 ms.
+// (the last also goes to the child that reaches furthest first; 201.0 M, 287 us
+// and 55 % of L1's whole throughput in the present build).  The frame: 1.455 ->
+// 1.283 ms; with 8 bounces 2.865 -> 2.550 ms.
 //
 // Nodes a walking lane visits per loop turn: with one 1.35, three 1.38
 // against 1.29 ms.
@@ -1770,9 +1770,11 @@ struct RoundLaunch {
 // frame): extend, then shadows and shading -- or, at a single frame's cache
 // depth, the cache gather.  Leaves `in` at the round's output queue.
 // Paths still bouncing at depth >= kTailDepth finish in the fused tail kernel
-// when the scene has no meshes.  With meshes the rounds stay: one thread per
-// remaining path would walk mesh BVHs and every light's shadow ray serially,
-// which on the config-2 scene took 1.8 ms against 1.3 ms for rounds 3-8.
+// when the scene has no meshes: textures at 1080p, depth 8, 394 us, with the
+// tail from depth 2 393 and from 4 419.  With meshes the rounds stay: one thread
+// per remaining path would walk mesh BVHs and every light's shadow ray serially
+// (1080p, 8 bounces, 2.88 against 1.99 ms; light meshes at 637x359 1.28 against
+// 0.69).
 constexpr uint32_t kTailDepth = 3;
 
 // The rest of the paths queued in `in` (depth `depth` on) in one fused kernel.
